@@ -20,6 +20,7 @@
 #include "flux.cuh"
 #include "fov_args.h"
 #include "internal.h"
+#include "pool_plan.h"
 
 namespace kb {
 
@@ -119,6 +120,7 @@ static int g_version = 0;
 static int g_skipped = 0;
 static std::map<int, DevState> g_dev;
 static EphemConst g_eph;  // host image of the constant table (pool pointer set per device)
+static PoolPlans g_plans;
 static std::vector<double> g_pool_host;
 static std::map<int64_t, int> g_slot_of;  // naif id -> slot
 
@@ -299,6 +301,96 @@ static void build_fast_plan(int n_force, FastPlan& P) {
     P.ok = (ok && n > 0 && lo <= hi) ? 1 : 0;
 }
 
+// The pooled kernels' series and bodies (PoolPlan) of the fast plan P: the same bodies,
+// centres, segments and window, with each series' records appended to the pool.
+static void build_pool_plan(const FastPlan& P, PoolPlan& Q) {
+    std::memset(&Q, 0, sizeof Q);
+    if (!P.ok) return;
+    std::map<int, int> at;  // SPK slot -> its position series
+    auto add_series = [&](int slot) {
+        if (at.count(slot)) return at[slot];
+        if (Q.n_pos >= MAX_SERIES) return -1;
+        const SegDesc& d = g_eph.seg[g_eph.slot[slot].first];
+        // trailing coefficients that are zero in every record (the padding of mixed counts)
+        // are left out
+        int nc = 2;
+        for (int64_t r = 0; r < d.n_rec; ++r)
+            for (int c = 0; c < 3; ++c)
+                for (int k = d.n_pad - 1; k >= nc; --k)
+                    if (g_pool_host[d.offset + r * d.rsize + 4 + c * d.n_pad + k] != 0.0) {
+                        nc = k + 1;
+                        break;
+                    }
+        const int pairs = (nc + 1) / 2;
+        if (g_pool_host.size() & 1) g_pool_host.push_back(0.0);
+        PoolSeries& S = Q.s[Q.n_pos];
+        S.offset = (int64_t)g_pool_host.size();
+        S.start_s = d.start_s;
+        S.inv_intlen = d.inv_intlen;
+        S.n_rec = d.n_rec;
+        S.rsize = 4 + 6 * pairs;
+        S.pairs = pairs;
+        S.slot = Q.n_slot;
+        g_pool_host.reserve(g_pool_host.size() + (size_t)d.n_rec * S.rsize);
+        for (int64_t r = 0; r < d.n_rec; ++r) {
+            const int64_t o = d.offset + r * d.rsize;
+            for (int64_t k : {o, o + 2, o + 3}) g_pool_host.push_back(g_pool_host[k]);
+            g_pool_host.push_back(0.0);
+            for (int j = 0; j < 2 * pairs; j += 2)
+                for (int c = 0; c < 3; ++c)
+                    for (int k = j; k < j + 2; ++k)
+                        g_pool_host.push_back(g_pool_host[o + 4 + c * d.n_pad + k]);
+        }
+        Q.n_slot += 3;
+        at[slot] = Q.n_pos;
+        return Q.n_pos++;
+    };
+    int vel_of[MAX_FORCE];
+    int centre = -1;
+    for (int it = 0; it < P.n_items; ++it) {
+        const FastItem& I = P.item[it];
+        if (I.role < 0) continue;
+        const int slot = g_eph.force[I.role].slot, parent = g_eph.slot[slot].parent_slot;
+        if (Q.n_body >= MAX_FORCE) return;
+        PoolBody& B = Q.b[Q.n_body];
+        const int pos = add_series(slot);
+        if (parent >= 0) centre = add_series(parent);
+        if (pos < 0 || (parent >= 0 && centre < 0)) return;
+        B.mass = I.mass;
+        B.radius = I.radius;
+        B.radius2 = I.radius * I.radius;
+        B.naif_id = I.naif_id;
+        B.kind = I.kind;
+        B.slot = Q.s[pos].slot;
+        B.chain = parent >= 0 ? Q.s[centre].slot : -1;
+        B.j2m = 1.5 * (I.kind == FK_SUN ? SUN_J2 : I.kind == FK_JUPITER ? JUPITER_J2
+                       : I.kind == FK_EARTH ? EARTH_J2 : 0.0) * I.mass;
+        if (it < P.n_vel) vel_of[Q.n_vel++] = pos;
+        ++Q.n_body;
+    }
+    // the kernels take the Sun first (the non-gravitational term is relative to it)
+    if (Q.n_vel != 2 || Q.b[0].kind != FK_SUN || Q.n_pos + Q.n_vel > MAX_SERIES ||
+        Q.n_body <= POOL_EARTH || Q.b[POOL_EARTH].kind != FK_EARTH)
+        return;
+    Q.n_series = Q.n_pos;
+    for (int v = 0; v < Q.n_vel; ++v) {
+        PoolSeries& S = Q.s[Q.n_series++];
+        S = Q.s[vel_of[v]];
+        S.slot = Q.b[v].vslot = Q.n_slot;
+        Q.n_slot += 3;
+    }
+    PoolBody& D = Q.b[Q.n_body];
+    D = Q.b[Q.n_body - 1];
+    D.mass = D.j2m = 0.0;
+    D.radius2 = -1.0;
+    D.kind = FK_PLAIN;
+    D.chain = -1;
+    // longest series first: the lanes of a warp then loop over similar counts
+    std::stable_sort(Q.s, Q.s + Q.n_pos,
+                     [](const PoolSeries& a, const PoolSeries& b) { return a.pairs > b.pairs; });
+    Q.ok = Q.n_slot <= POOL_MAX_SLOTS ? 1 : 0;
+}
+
 // Build the slot / segment / force tables and the device record pool from g_segs.
 static int rebuild_tables() {
     std::memset(&g_eph, 0, sizeof g_eph);
@@ -437,6 +529,8 @@ static int rebuild_tables() {
     g_eph.n_force_all = (planets_ok && all_ok) ? N_MASSES : 0;
     build_fast_plan(g_eph.n_force_planets, g_eph.fast_planets);
     build_fast_plan(g_eph.n_force_all, g_eph.fast_all);
+    build_pool_plan(g_eph.fast_planets, g_plans.planets);
+    build_pool_plan(g_eph.fast_all, g_plans.all);
     g_eph.sun_slot = g_slot_of.count(10) ? g_slot_of[10] : -1;
     g_eph.loaded = 1;
     ++g_version;
@@ -582,7 +676,7 @@ static int ensure_device(DevState*& out) {
             return rc;
         EphemConst e = g_eph;
         e.pool = ds.pool;
-        if ((rc = upload_ephem(e))) return rc;
+        if ((rc = upload_ephem(e)) || (rc = upload_pool_plans(g_plans))) return rc;
         ds.version = g_version;
     }
     out = &ds;
@@ -673,10 +767,31 @@ struct Stager {
 int nodes_variant_for(int variant, int n_force) {
     if (variant < 6) return variant;
     const FastPlan& P = n_force == g_eph.n_force_planets ? g_eph.fast_planets : g_eph.fast_all;
-    if (variant >= 9)  // pooled: the uncached step-end form of the same register budget
-        return (!P.ok || pool_plan_doubles(P) > POOL_CACHE_DOUBLES) ? variant - 5 : variant;
+    if (variant >= 9) {  // pooled: the uncached step-end form of the same register budget
+        const PoolPlan& Q =
+            n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
+        return Q.ok ? variant : variant - 5;
+    }
     if (!P.ok || fast_plan_cache_doubles(P) > EPH_CACHE) return variant - 3;
     return variant;
+}
+
+// The form a call in the automatic mode runs while the launch configuration is the one the
+// library starts with.  All of them give the same results to the bit; which is faster was
+// measured on B200 with the main belt over one year (us):
+//   n            1    600   2368   4000   10000   64000
+//   wide       144    271    379    528    1150    6240
+//   variant 9  197    456    475    579     746    3533   (168 registers, refill)
+//   variant 10 209    513    542    664     836    3545   (128 registers, refill)
+// A warp per object is the shortest wait until the warps fill the GPU twice; above, four
+// objects share a warp, and the 128-register form's extra warps pay once the queue holds many
+// objects per lane group (a +-5 yr mix of 125,000: 16.5 ms against 17.8; a million: 125.0
+// against 135.8).
+constexpr int64_t AUTO_WIDE_MAX = 4096, AUTO_168_MAX = 98304;
+static int auto_variant(int64_t n, int n_force) {
+    const PoolPlan& Q = n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
+    if (!Q.ok) return nodes_variant_for(7, n_force);
+    return n <= AUTO_WIDE_MAX ? NODES_WIDE : n <= AUTO_168_MAX ? 9 : 10;
 }
 
 // The window a variant needs its objects' spans inside (the warp-pooled kernels: the fast
@@ -691,9 +806,23 @@ void nodes_window(int variant, int n_force, double& lo, double& hi) {
     }
 }
 
+// Whether the launch configuration is the one the library starts with.
+static bool launch_is_default() {
+    const LaunchConfig d;
+    return g_launch.nodes_variant == d.nodes_variant && g_launch.nodes_refill == d.nodes_refill;
+}
+
+// What the pooled kernels read besides the plan in constant memory.
+static void set_pool(NBodyArgs& a, double lo, double hi) {
+    const PoolPlan& Q = a.n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
+    a.pool_slots = Q.n_slot;
+    a.lo = lo;
+    a.hi = hi;
+}
+
 // Everything the allocation-free entry point needs, read under the lock without allocating:
 // the ephemeris must already be resident on the current device.
-int noalloc_snapshot(int include_asteroids, int64_t center, NBodyArgs& a, LaunchConfig& cfg,
+int noalloc_snapshot(int64_t n, int include_asteroids, int64_t center, NBodyArgs& a, LaunchConfig& cfg,
                      NodesPlan& plan) {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!g_eph.loaded) return set_error(KETE_B200_E_NO_EPHEMERIS, "no SPK loaded");
@@ -711,9 +840,11 @@ int noalloc_snapshot(int include_asteroids, int64_t center, NBodyArgs& a, Launch
     if ((rc = center_chain(center, a.chain))) return rc;
     a.n_force = n_force;
     cfg = g_launch;
-    cfg.nodes_variant = nodes_variant_for(cfg.nodes_variant, n_force);
+    cfg.nodes_variant = launch_is_default() ? auto_variant(n, n_force)
+                                            : nodes_variant_for(cfg.nodes_variant, n_force);
     plan.general_variant = nodes_variant_for(7, n_force);
     nodes_window(cfg.nodes_variant, n_force, plan.lo, plan.hi);
+    set_pool(a, plan.lo, plan.hi);
     return 0;
 }
 
@@ -950,20 +1081,30 @@ int kete_b200_propagate_n_body(int64_t n, const double* pos, const double* vel, 
     if (mode == KETE_B200_MODE_THREAD) {
         if ((rc = launch_nbody_thread(a, g_launch.thread_block, st))) return rc;
     } else if (mode == KETE_B200_MODE_NODES || mode == KETE_B200_MODE_AUTO) {
+        const bool automatic = mode == KETE_B200_MODE_AUTO && launch_is_default();
+        const int variant = automatic ? auto_variant(n, a.n_force)
+                                      : nodes_variant_for(g_launch.nodes_variant, a.n_force);
+        const bool refill = automatic ? variant >= 9 : g_launch.nodes_refill != 0;
+        double lo, hi;
+        nodes_window(variant, a.n_force, lo, hi);
+        set_pool(a, lo, hi);
+        if (variant == NODES_WIDE) {
+            if ((rc = launch_nodes_wide(a, nodes_variant_for(7, a.n_force), st))) return rc;
+            return S.finish();
+        }
         // objects in order of their work (span in orbital periods), most first; scratch holds
         // the queue counter, the work histogram and the processing order
         void* q = nullptr;
         if ((rc = staging(*ds, 31, (ORDER_SCRATCH_HEADER + (size_t)n) * sizeof(int), &q)))
             return rc;
-        const int variant = nodes_variant_for(g_launch.nodes_variant, a.n_force);
-        double lo, hi;
-        nodes_window(variant, a.n_force, lo, hi);
+        int groups = 0;
+        if ((rc = pool_groups(variant, n, a.pool_slots, refill, &groups))) return rc;
         if ((rc = launch_span_order(n, a.pos, a.vel, a.jd0, a.jd1, lo, hi,
-                                    variant >= 9 ? a.nongrav : nullptr, (int*)q, st)))
+                                    variant >= 9 ? a.nongrav : nullptr, groups, (int*)q, st)))
             return rc;
         // refill: a persistent grid taking the next object from the queue
         if ((rc = launch_nodes_ordered(a, variant, nodes_variant_for(7, a.n_force),
-                                       g_launch.nodes_refill != 0, (int*)q, st)))
+                                       refill, (int*)q, st)))
             return rc;
     } else {
         return set_error(KETE_B200_E_ARGUMENT, "unknown propagation mode");

@@ -17,6 +17,7 @@ enum Status : int32_t {
     ST_IO_ERROR = 5,
     ST_IMPACT = 6,
     ST_TIMEOUT = 7,  // a bounded device loop ran out of iterations
+    ST_PENDING = -1,  // internal: left by one kernel of a call to the next
     ST_CHECKPOINT_FULL = 8,  // more checkpoints were needed than the caller provided
 };
 

@@ -21,20 +21,22 @@ constexpr int MAX_SLOT = 32;
 constexpr int MAX_FORCE = 16;
 constexpr int MAX_CHAIN = 3;
 // span ordering of the persistent N-body grid: work buckets, and the scratch header (ints):
-// [0] object queue, [1 ..] bucket histogram, then the bucket cursors (ORDER_BUCKETS work
-// buckets, then one bucket for the objects with a non-gravitational model and one for the
-// objects whose span leaves the fast plan's window; the first two kinds only when the caller
-// asks for the split), ORDER_RANGE: {0, start of the non-gravitational bucket, start of the
-// outside bucket, n}, ORDER_QUEUE2: the queue of the objects outside the window,
-// ORDER_QUEUE3: the queue of the non-gravitational bucket; the processing order follows the
-// header
-constexpr int ORDER_BUCKETS = 120;
-constexpr int ORDER_NG_BUCKET = ORDER_BUCKETS;
-constexpr int ORDER_OUT_BUCKET = ORDER_BUCKETS + 1;
-constexpr int ORDER_ALL_BUCKETS = ORDER_BUCKETS + 2;
+// [0] object queue, [1 ..] bucket histogram, then the bucket cursors; ORDER_RANGE: {0, start of
+// the non-gravitational buckets, start of the outside bucket, n}, ORDER_QUEUE2: the queue of
+// the objects outside the window, ORDER_QUEUE3: the queue of the non-gravitational part; the
+// processing order follows the header.  Buckets: ORDER_CLASSES work classes, the same classes
+// again for the objects with a non-gravitational model, and one for the objects whose span
+// leaves the fast plan's window (the last two kinds only when the caller asks for the split).
+constexpr int ORDER_CLASSES = 60;
+constexpr int ORDER_NG_BUCKET = ORDER_CLASSES;
+constexpr int ORDER_OUT_BUCKET = 2 * ORDER_CLASSES;
+constexpr int ORDER_ALL_BUCKETS = ORDER_OUT_BUCKET + 1;
 constexpr int ORDER_RANGE = 1 + 2 * ORDER_ALL_BUCKETS;
 constexpr int ORDER_QUEUE2 = ORDER_RANGE + 4;
 constexpr int ORDER_QUEUE3 = ORDER_RANGE + 5;
+// ORDER_WIDE: {heavy objects leading the first part, leading the non-gravitational part, their
+// queue}; the other two queues start behind them
+constexpr int ORDER_WIDE = ORDER_RANGE + 6;
 constexpr int EPH_CACHE = 38;  // body-position cache, doubles per lane (the planets need 36)
 
 constexpr int ORDER_SCRATCH_HEADER = 256;
@@ -111,18 +113,6 @@ struct FastPlan {
     FastItem item[MAX_ITEMS];
 };
 
-// Body cache of the warp-pooled node kernel (radau_pool.cuh), doubles per lane: position and
-// velocity of the first n_vel items, positions of every other item but padding (centres
-// included: the bodies chained to them add the centre's position when the force terms read
-// them).  The planets need 39.
-constexpr int POOL_CACHE_DOUBLES = 40;
-inline __host__ __device__ int pool_plan_doubles(const FastPlan& P) {
-    int k = 6 * P.n_vel;
-    for (int it = P.n_vel; it < P.n_items; ++it)
-        if (P.item[it].role != -2) k += 3;
-    return k;
-}
-
 // Doubles a lane's body-position cache needs for a fast plan (SpkForceT::fast_positions):
 // position and velocity of the first n_vel bodies, positions of the other force bodies.
 inline __host__ __device__ int fast_plan_cache_doubles(const FastPlan& P) {
@@ -142,6 +132,12 @@ struct EphemConst {
     ForceEntry force[MAX_FORCE];
     const double* pool;
 };
+
+// Whether a Radau integration from jd0 to jd1 stays inside the window [lo, hi].
+__device__ __forceinline__ bool in_window(double jd0, double jd1, double lo, double hi) {
+    constexpr double MARGIN = 1e-6;  // NaN epochs compare false: outside
+    return jd0 >= lo + MARGIN && jd1 >= lo + MARGIN && jd0 <= hi - MARGIN && jd1 <= hi - MARGIN;
+}
 
 // Evaluate one record: position (AU) and velocity (AU/day) of the segment's body.
 __device__ __forceinline__ void cheb_record(const double* __restrict__ rec, int n_coef, int n_pad,

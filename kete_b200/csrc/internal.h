@@ -39,6 +39,7 @@ int upload_tables(const Tables& t);
 int upload_ephem(const EphemConst& e);
 int upload_consts_kernels(const Tables* t, const EphemConst* e);
 int upload_consts_nodes(const Tables* t, const EphemConst* e);
+int upload_consts_pool(const Tables* t, const EphemConst* e);
 int upload_consts_sens(const Tables* t, const EphemConst* e);
 int upload_consts_adjoint(const Tables* t, const EphemConst* e);
 int upload_consts_long(const Tables* t, const EphemConst* e);
@@ -67,6 +68,11 @@ struct NBodyArgs {
                           // (null: order[0 .. n)); the pooled kernel: {first, start of the
                           // non-gravitational part, end}
     int* queue_ng;        // pooled kernel with refill: the queue of the non-gravitational part
+    int* wide;            // pooled kernels: {heavy objects leading the order's first part, those
+                          // leading its non-gravitational part, the queue of both}
+    int pool_slots;       // pooled kernels: doubles of a cache column (PoolPlan::n_slot)
+    double lo, hi;        // wide pooled kernel: the fast plan's window
+    int pending;          // node kernel: only the objects whose status is ST_PENDING
 };
 
 int launch_two_body(int64_t n, const double* pos, const double* vel, const double* jd0,
@@ -80,16 +86,26 @@ int launch_covariance(int64_t n, int rows, int cols, const double* phi, const do
                       double* out, cudaStream_t stream);
 int launch_nbody_thread(const NBodyArgs& a, int block, cudaStream_t stream);
 int launch_nbody_nodes(const NBodyArgs& a, int variant, int grid, cudaStream_t stream);
-int nodes_grid_size(int variant, int* grid);
+// pool.cu: the warp-pooled kernels' entry, shared memory, launch, and the centre changes of
+// their objects before and after it
+const void* pool_kernel_ptr(int variant);
+int pool_smem(int variant, int slots, int* bytes);
+int launch_pool(const NBodyArgs& a, int variant, int grid, cudaStream_t stream);
+int launch_pool_centre(const NBodyArgs& a, bool before, cudaStream_t stream);
+int nodes_grid_size(int variant, int slots, int* grid);
+// lane groups that a variant's persistent grid has for n objects (0: not a pooled variant with
+// refill), for launch_span_order's choice of the heavy objects
+int pool_groups(int variant, int64_t n, int slots, bool refill, int* groups);
 // load the node kernels and the processing-order kernels into the current context (module
 // loading is lazy: done here, it does not happen inside a later call)
 int preload_nodes_kernels();
+int preload_pool_kernels();
 int preload_order_kernels();
 // resolve the allocation-free entry point's scratch address on the current device
 int noalloc_prepare();
 int launch_span_order(int64_t n, const double* pos, const double* vel, const double* jd0,
-                      const double* jd1, double lo, double hi, const double* ng, int* scratch,
-                      cudaStream_t stream);
+                      const double* jd1, double lo, double hi, const double* ng, int groups,
+                      int* scratch, cudaStream_t stream);
 // The node kernels over the processing order that launch_span_order wrote into scratch
 // (variant as launch_nbody_nodes; refill: persistent grid with the object queue).  A
 // warp-pooled variant integrates the objects inside the fast plan's window (those with a
@@ -98,6 +114,11 @@ int launch_span_order(int64_t n, const double* pos, const double* vel, const dou
 // variant takes the whole order in one launch.
 int launch_nodes_ordered(NBodyArgs a, int variant, int general_variant, bool refill,
                          int* scratch, cudaStream_t stream);
+
+// The wide pooled kernel (a warp per object) over every object in the caller's order, then
+// general_variant over those whose span leaves the fast plan's window.
+constexpr int NODES_WIDE = 11;  // internal variant number: not a launch configuration
+int launch_nodes_wide(NBodyArgs a, int general_variant, cudaStream_t stream);
 
 // launch configuration chosen by the tuner (kete_b200_set_launch_config)
 struct LaunchConfig {
@@ -121,7 +142,7 @@ struct NodesPlan {
     int general_variant;
     double lo, hi;
 };
-int noalloc_snapshot(int include_asteroids, int64_t center, NBodyArgs& a, LaunchConfig& cfg,
+int noalloc_snapshot(int64_t n, int include_asteroids, int64_t center, NBodyArgs& a, LaunchConfig& cfg,
                      NodesPlan& plan);
 int launch_radau_central(int64_t n, const double* pos, const double* vel, const double* t0,
                          const double* t1, double* out_pos, double* out_vel, int32_t* status,

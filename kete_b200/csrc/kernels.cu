@@ -24,15 +24,15 @@ KB_CONSTANT_UPLOADER(kernels)
 
 int upload_tables(const Tables& t) {
     int rc = 0;
-    for (auto up : {upload_consts_kernels, upload_consts_nodes, upload_consts_sens,
-                    upload_consts_adjoint, upload_consts_long})
+    for (auto up : {upload_consts_kernels, upload_consts_nodes, upload_consts_pool,
+                    upload_consts_sens, upload_consts_adjoint, upload_consts_long})
         if ((rc = up(&t, nullptr))) return rc;
     return 0;
 }
 int upload_ephem(const EphemConst& e) {
     int rc = 0;
-    for (auto up : {upload_consts_kernels, upload_consts_nodes, upload_consts_sens,
-                    upload_consts_adjoint, upload_consts_long})
+    for (auto up : {upload_consts_kernels, upload_consts_nodes, upload_consts_pool,
+                    upload_consts_sens, upload_consts_adjoint, upload_consts_long})
         if ((rc = up(nullptr, &e))) return rc;
     return 0;
 }
@@ -284,29 +284,21 @@ namespace kb {
 // the orbit.  With a persistent grid the groups that finish early pick up the small ones
 // and the tail is short; with one group per object, neighbours in a warp get similar work,
 // so the warp-synchronous forms' groups wait less for each other.  Work is bucketed on a
-// log2 scale (quarter-octave classes from 2^-8 to 2^7 radians, each split by the direction
-// of integration); within a bucket the order is whatever the atomics give -- it does not
-// affect any object's result.
+// log2 scale (quarter-octave classes from 2^-8 to 2^7 radians); within a bucket the order is
+// whatever the atomics give -- it does not affect any object's result.
 //
 // The warp-pooled node kernel evaluates the ephemeris from the fast plan's records alone, so
 // the objects whose span [jd0, jd1] does not lie inside the plan's window (with a margin of
 // 1e-6 day: every evaluation time of a Radau integration lies between jd0 and jd1 up to
-// rounding) go to one last bucket.  Before it, one bucket holds the objects with a
-// non-gravitational model (given ng), which the pooled kernel integrates on a few SMs of
-// their own: the model's code, fetched by any warp of an SM, evicts the step loop from the
-// SM's instruction cache.  The header's range {0, ng start, outside start, n} splits the
-// order.  Callers without a window pass [-inf, inf] and ng = null.
-//
-// Scratch layout (ints): [0] object queue, [1..ORDER_ALL_BUCKETS] bucket histogram, then the
-// bucket cursors, the range at ORDER_RANGE, further queues at ORDER_QUEUE2 and ORDER_QUEUE3,
-// then order[n] from int offset ORDER_SCRATCH_HEADER.
+// rounding) go to one last bucket.  Before it, the objects with a non-gravitational model (given
+// ng) have the work classes to themselves: the pooled kernel integrates them on a few SMs of
+// their own (the model's code, fetched by any warp of an SM, evicts the step loop from the
+// SM's instruction cache), also most work first.  (In one bucket, unsorted, their long ones
+// started late: 100,000 objects of the +-5 yr mix took 19.6 ms with a third of the SM time
+// idle at the end.)  The header's range {0, ng start, outside start, n} splits the order.
+// Callers without a window pass [-inf, inf] and ng = null.
 // -------------------------------------------------------------------------------------------
-static_assert(ORDER_QUEUE3 + 1 <= ORDER_SCRATCH_HEADER, "order header too small");
-
-__device__ __forceinline__ bool in_window(double jd0, double jd1, double lo, double hi) {
-    constexpr double MARGIN = 1e-6;  // NaN epochs compare false: outside
-    return jd0 >= lo + MARGIN && jd1 >= lo + MARGIN && jd0 <= hi - MARGIN && jd1 <= hi - MARGIN;
-}
+static_assert(ORDER_WIDE + 3 <= ORDER_SCRATCH_HEADER, "order header too small");
 
 __device__ __forceinline__ int work_bucket(int64_t i, int64_t n, const double* __restrict__ pos,
                                            const double* __restrict__ vel, double jd0, double jd1) {
@@ -317,23 +309,16 @@ __device__ __forceinline__ int work_bucket(int64_t i, int64_t n, const double* _
     const double inv_a = 2.0 / r - (vx * vx + vy * vy + vz * vz) / GMS;
     const double mean_motion = inv_a > 0.0 ? sqrt(GMS * inv_a * inv_a * inv_a) : sqrt(GMS / (r * r * r));
     const double work = span * mean_motion;
-    if (!(work > 0.0) || !isfinite(work)) return ORDER_BUCKETS - 1;  // no work, NaN last
-    // quarter-octave work classes, most work first; within a class the objects integrated
-    // forwards in time come before those integrated backwards, so that neighbours in the
-    // order (the lane groups of a warp, the groups of a block) also move through the
-    // ephemeris in the same direction and share more of its records
-    constexpr int CLASSES = ORDER_BUCKETS / 2;
+    if (!(work > 0.0) || !isfinite(work)) return ORDER_CLASSES - 1;  // no work, NaN last
     const int b = (int)floor(log2(work) * 4.0) + 32;
-    const int cls = CLASSES - 1 - (b < 0 ? 0 : (b > CLASSES - 1 ? CLASSES - 1 : b));
-    return 2 * cls + (jd1 < jd0 ? 1 : 0);
+    return ORDER_CLASSES - 1 - (b < 0 ? 0 : (b > ORDER_CLASSES - 1 ? ORDER_CLASSES - 1 : b));
 }
 
 __device__ __forceinline__ int order_bucket(int64_t i, int64_t n, const double* __restrict__ pos,
                                             const double* __restrict__ vel, double t0, double t1,
                                             double lo, double hi, const double* __restrict__ ng) {
     if (!in_window(t0, t1, lo, hi)) return ORDER_OUT_BUCKET;
-    if (ng && ng[i] != 0.0) return ORDER_NG_BUCKET;
-    return work_bucket(i, n, pos, vel, t0, t1);
+    return work_bucket(i, n, pos, vel, t0, t1) + (ng && ng[i] != 0.0 ? ORDER_NG_BUCKET : 0);
 }
 
 __global__ void order_hist_kernel(int64_t n, const double* __restrict__ pos,
@@ -351,30 +336,83 @@ __global__ void order_hist_kernel(int64_t n, const double* __restrict__ pos,
         if (h[i]) atomicAdd(&scratch[1 + i], h[i]);
 }
 
-__global__ void order_scan_kernel(int* __restrict__ scratch) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        int run = 0;
-        for (int b = 0; b < ORDER_ALL_BUCKETS; ++b) {
-            if (b == ORDER_NG_BUCKET) scratch[ORDER_RANGE + 1] = run;
-            if (b == ORDER_OUT_BUCKET) scratch[ORDER_RANGE + 2] = run;  // objects inside the window
-            scratch[1 + ORDER_ALL_BUCKETS + b] = run;
-            run += scratch[1 + b];
-        }
+constexpr int ORDER_BLOCK = 256;
+
+// Bucket starts (the cursors) and the range from the histogram: one block, one bucket a thread.
+//
+// groups > 0 (a persistent pooled launch with that many lane groups): the objects of the classes
+// whose work is over HEAVY_SHARE of a group's share of all the work would still run when the
+// others are done; the pooled kernel gives them a warp each (at most half its warps' worth).
+constexpr float HEAVY_SHARE = 1.0f;
+__global__ void __launch_bounds__(ORDER_BLOCK) order_scan_kernel(int groups,
+                                                                 int* __restrict__ scratch) {
+    __shared__ int start[ORDER_BLOCK];
+    __shared__ float total;
+    const int t = threadIdx.x;
+    const int own = t < ORDER_ALL_BUCKETS ? scratch[1 + t] : 0;
+    start[t] = own;
+    __syncthreads();
+    for (int o = 1; o < ORDER_BLOCK; o <<= 1) {  // inclusive sums
+        const int v = t >= o ? start[t - o] : 0;
+        __syncthreads();
+        start[t] += v;
+        __syncthreads();
+    }
+    if (t < ORDER_ALL_BUCKETS) scratch[1 + ORDER_ALL_BUCKETS + t] = start[t] - own;
+    if (t == 0) {
         scratch[ORDER_RANGE] = 0;
-        scratch[ORDER_RANGE + 3] = run;
+        scratch[ORDER_RANGE + 1] = start[ORDER_NG_BUCKET - 1];
+        scratch[ORDER_RANGE + 2] = start[ORDER_OUT_BUCKET - 1];
+        scratch[ORDER_RANGE + 3] = start[ORDER_OUT_BUCKET];
+        total = 0.0f;
+    }
+    if (groups <= 0) return;
+    __syncthreads();
+    const int cls = t < ORDER_NG_BUCKET ? t : t - ORDER_NG_BUCKET;
+    const float work = exp2f((float)(ORDER_CLASSES - 1 - 32 - cls) * 0.25f);  // the class's least
+    if (t < ORDER_OUT_BUCKET) atomicAdd(&total, (float)own * work * 1.09f);
+    __syncthreads();
+    if (t == 0 || t == ORDER_NG_BUCKET) {
+        const float limit = HEAVY_SHARE * total / (float)groups;
+        const int most = groups / 16;  // of each part: a quarter of the warps
+        int heavy = 0;
+        for (int c = 0; c < ORDER_CLASSES; ++c) {
+            const int add = scratch[1 + t + c];
+            if (exp2f((float)(ORDER_CLASSES - 1 - 32 - c) * 0.25f) <= limit || heavy + add > most) break;
+            heavy += add;
+        }
+        scratch[ORDER_WIDE + (t ? 1 : 0)] = heavy;
+        scratch[t ? ORDER_QUEUE3 : 0] = heavy;
     }
 }
 
-__global__ void order_scatter_kernel(int64_t n, const double* __restrict__ pos,
-                                     const double* __restrict__ vel, const double* __restrict__ jd0,
-                                     const double* __restrict__ jd1, double lo, double hi,
-                                     const double* __restrict__ ng, int* __restrict__ scratch,
-                                     int32_t* __restrict__ order) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        const int b = order_bucket(i, n, pos, vel, jd0[i], jd1[i], lo, hi, ng);
-        const int p = atomicAdd(&scratch[1 + ORDER_ALL_BUCKETS + b], 1);
-        if (p >= 0 && p < n) order[p] = (int32_t)i;
+// Tiles of one object per thread: ranks inside a tile come from shared-memory counters and a
+// tile takes its place in each bucket with one global atomic (one per object on a few hot
+// cursors took 223 us on 1M objects).
+__global__ void __launch_bounds__(ORDER_BLOCK) order_scatter_kernel(
+    int64_t n, const double* __restrict__ pos, const double* __restrict__ vel,
+    const double* __restrict__ jd0, const double* __restrict__ jd1, double lo, double hi,
+    const double* __restrict__ ng, int* __restrict__ scratch, int32_t* __restrict__ order) {
+    __shared__ int count[ORDER_ALL_BUCKETS], base[ORDER_ALL_BUCKETS];
+    const int t = threadIdx.x;
+    for (int64_t first = (int64_t)blockIdx.x * ORDER_BLOCK; first < n;
+         first += (int64_t)gridDim.x * ORDER_BLOCK) {
+        if (t < ORDER_ALL_BUCKETS) count[t] = 0;
+        __syncthreads();
+        const int64_t i = first + t;
+        int b = 0, rank = 0;
+        if (i < n) {
+            b = order_bucket(i, n, pos, vel, jd0[i], jd1[i], lo, hi, ng);
+            rank = atomicAdd(&count[b], 1);
+        }
+        __syncthreads();
+        if (t < ORDER_ALL_BUCKETS && count[t])
+            base[t] = atomicAdd(&scratch[1 + ORDER_ALL_BUCKETS + t], count[t]);
+        __syncthreads();
+        if (i < n) {
+            const int p = base[b] + rank;
+            if (p >= 0 && p < n) order[p] = (int32_t)i;
+        }
     }
 }
 
@@ -392,18 +430,17 @@ int preload_order_kernels() {
 // plan's window whose outsiders are ordered last, ng: the non-gravitational rows whose
 // objects are ordered just before them ([-inf, inf] and null: no split).
 int launch_span_order(int64_t n, const double* pos, const double* vel, const double* jd0,
-                      const double* jd1, double lo, double hi, const double* ng, int* scratch,
-                      cudaStream_t stream) {
+                      const double* jd1, double lo, double hi, const double* ng, int groups,
+                      int* scratch, cudaStream_t stream) {
     int rc = cuda_check(cudaMemsetAsync(scratch, 0, ORDER_SCRATCH_HEADER * sizeof(int), stream),
                         "clear order header");
     if (rc || n <= 0) return rc;
-    const int block = 256;
-    int64_t g = (n + block - 1) / block;
+    const int64_t g = (n + ORDER_BLOCK - 1) / ORDER_BLOCK;
     const int grid = (int)(g > 1184 ? 1184 : g);
-    order_hist_kernel<<<grid, block, 0, stream>>>(n, pos, vel, jd0, jd1, lo, hi, ng, scratch);
-    order_scan_kernel<<<1, 32, 0, stream>>>(scratch);
-    order_scatter_kernel<<<grid, block, 0, stream>>>(n, pos, vel, jd0, jd1, lo, hi, ng, scratch,
-                                                     (int32_t*)(scratch + ORDER_SCRATCH_HEADER));
+    order_hist_kernel<<<grid, ORDER_BLOCK, 0, stream>>>(n, pos, vel, jd0, jd1, lo, hi, ng, scratch);
+    order_scan_kernel<<<1, ORDER_BLOCK, 0, stream>>>(groups, scratch);
+    order_scatter_kernel<<<grid, ORDER_BLOCK, 0, stream>>>(
+        n, pos, vel, jd0, jd1, lo, hi, ng, scratch, (int32_t*)(scratch + ORDER_SCRATCH_HEADER));
     return launched(3, "span order launch");
 }
 

@@ -88,7 +88,7 @@ extern "C" int kete_b200_propagate_n_body_noalloc(
     std::memset(&a, 0, sizeof a);
     LaunchConfig cfg;
     NodesPlan plan;
-    int rc = noalloc_snapshot(include_asteroids, center, a, cfg, plan);
+    int rc = noalloc_snapshot(n, include_asteroids, center, a, cfg, plan);
     if (rc) return rc;
     int* scratch = nullptr;
     if ((rc = noalloc_scratch(&scratch))) return rc;
@@ -109,8 +109,11 @@ extern "C" int kete_b200_propagate_n_body_noalloc(
     a.min_dist = min_dist;
     a.counters = counters;
     a.max_loops = cfg.max_loops;
+    if (cfg.nodes_variant == NODES_WIDE) return launch_nodes_wide(a, plan.general_variant, st);
+    int groups = 0;
+    if ((rc = pool_groups(cfg.nodes_variant, n, a.pool_slots, true, &groups))) return rc;
     if ((rc = launch_span_order(n, pos, vel, jd0, jd1, plan.lo, plan.hi,
-                                cfg.nodes_variant >= 9 ? nongrav : nullptr, scratch, st)))
+                                cfg.nodes_variant >= 9 ? nongrav : nullptr, groups, scratch, st)))
         return rc;
     return launch_nodes_ordered(a, cfg.nodes_variant, plan.general_variant, true, scratch, st);
 }

@@ -1,17 +1,13 @@
-// nodes.cu -- host launchers of the node-parallel Radau kernels (radau_nodes.cuh and the
-// warp-pooled form of radau_pool.cuh): every register-cap / step-end / warp-synchronous /
+// nodes.cu -- host launchers of the node-parallel Radau kernels (radau_nodes.cuh here, the
+// warp-pooled forms in pool.cu): every register-cap / step-end / warp-synchronous /
 // pooled instantiation the tuner chooses from.  Its own translation unit so the
 // instantiations compile in parallel with the other kernels.
-#include <algorithm>
-#include <atomic>
-
 #include "../../include/kete_b200.h"
 
 #include "common.cuh"
 #include "forces.cuh"
 #include "internal.h"
 #include "radau_nodes.cuh"
-#include "radau_pool.cuh"
 
 namespace kb {
 KB_CONSTANT_UPLOADER(nodes)
@@ -27,8 +23,9 @@ namespace kb {
 // 9, 10: the warp-pooled record evaluations (radau_pool.cuh) at 168 / 128 registers.
 static const void* nodes_kernel_ptr(int variant) {
     switch (variant) {
-        case 9: return (const void*)nbody_pool_kernel<3>;
-        case 10: return (const void*)nbody_pool_kernel<4>;
+        case NODES_WIDE:
+        case 9:
+        case 10: return pool_kernel_ptr(variant);
         case 1: return (const void*)nbody_nodes_kernel<3, false>;
         case 2: return (const void*)nbody_nodes_kernel<4, false>;
         case 3: return (const void*)nbody_nodes_kernel<1, true>;
@@ -41,28 +38,6 @@ static const void* nodes_kernel_ptr(int variant) {
     }
 }
 
-static int dyn_smem(int variant) { return variant >= 9 ? POOL_DYN_SMEM : 0; }
-
-// The pooled kernels keep their body cache in dynamic shared memory above the 48 KB static
-// limit: allow it once per device (a function attribute, not a stream operation).
-static int allow_dyn_smem(int variant) {
-    static std::atomic<unsigned long long> done[2];
-    if (variant < 9) return 0;
-    int dev = 0;
-    int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    if (rc) return rc;
-    const unsigned long long bit = 1ull << (dev & 63);
-    auto& d = done[variant - 9];
-    if (d.load() & bit) return 0;
-    if ((rc = cuda_check(cudaFuncSetAttribute(nodes_kernel_ptr(variant),
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              dyn_smem(variant)),
-                         "pooled kernel shared memory")))
-        return rc;
-    d.fetch_or(bit);
-    return 0;
-}
-
 int launch_nbody_nodes(const NBodyArgs& a, int variant, int grid, cudaStream_t stream) {
     if (a.n <= 0) return 0;
     if (variant >= 9 && !a.range)
@@ -71,11 +46,8 @@ int launch_nbody_nodes(const NBodyArgs& a, int variant, int grid, cudaStream_t s
                          "order (launch_nodes_ordered)");
     const int block = NODES_BLOCK;
     if (grid <= 0) grid = (int)((a.n * NODE_G + block - 1) / block);
-    int rc = allow_dyn_smem(variant);
-    if (rc) return rc;
+    if (variant >= 9) return launch_pool(a, variant, grid, stream);
     switch (variant) {
-        case 9: nbody_pool_kernel<3><<<grid, block, POOL_DYN_SMEM, stream>>>(a); break;
-        case 10: nbody_pool_kernel<4><<<grid, block, POOL_DYN_SMEM, stream>>>(a); break;
         case 1: nbody_nodes_kernel<3, false><<<grid, block, 0, stream>>>(a); break;
         case 2: nbody_nodes_kernel<4, false><<<grid, block, 0, stream>>>(a); break;
         case 3: nbody_nodes_kernel<1, true><<<grid, block, 0, stream>>>(a); break;
@@ -90,12 +62,21 @@ int launch_nbody_nodes(const NBodyArgs& a, int variant, int grid, cudaStream_t s
 }
 
 // Persistent grid of a variant, capped at one lane group per object.
-static int refill_grid(int variant, int64_t n, int* grid) {
-    int rc = nodes_grid_size(variant, grid);
+static int refill_grid(int variant, int64_t n, int slots, int* grid) {
+    int rc = nodes_grid_size(variant, slots, grid);
     if (rc) return rc;
     const int64_t need = (n * NODE_G + NODES_BLOCK - 1) / NODES_BLOCK;
     if (*grid > need) *grid = (int)need;
     return 0;
+}
+
+int pool_groups(int variant, int64_t n, int slots, bool refill, int* groups) {
+    *groups = 0;
+    if (variant < 9 || !refill) return 0;
+    int grid = 0;
+    const int rc = refill_grid(variant, n, slots, &grid);
+    *groups = grid * (NODES_BLOCK / NODE_G);
+    return rc;
 }
 
 int launch_nodes_ordered(NBodyArgs a, int variant, int general_variant, bool refill,
@@ -105,7 +86,7 @@ int launch_nodes_ordered(NBodyArgs a, int variant, int general_variant, bool ref
     if (variant < 9) {  // one launch over the whole order
         a.range = nullptr;
         a.queue = refill ? scratch : nullptr;
-        if (refill && (rc = refill_grid(variant, a.n, &grid))) return rc;
+        if (refill && (rc = refill_grid(variant, a.n, a.pool_slots, &grid))) return rc;
         return launch_nbody_nodes(a, variant, grid, stream);
     }
     // objects inside the window: the pooled kernel between its centre-change kernels; the
@@ -114,44 +95,49 @@ int launch_nodes_ordered(NBodyArgs a, int variant, int general_variant, bool ref
     a.range = scratch + ORDER_RANGE;
     a.queue = refill ? scratch : nullptr;
     a.queue_ng = refill ? scratch + ORDER_QUEUE3 : nullptr;
-    const int64_t cgrid = std::min<int64_t>((a.n + 255) / 256, 1184);
-    pool_prepare_kernel<<<(int)cgrid, 256, 0, stream>>>(a);
-    if ((rc = launched(1, "pool_prepare_kernel launch"))) return rc;
-    if (refill && (rc = refill_grid(variant, a.n, &grid))) return rc;
+    a.wide = scratch + ORDER_WIDE;
+    if ((rc = launch_pool_centre(a, true, stream))) return rc;
+    if (refill && (rc = refill_grid(variant, a.n, a.pool_slots, &grid))) return rc;
     if ((rc = launch_nbody_nodes(a, variant, grid, stream))) return rc;
-    pool_finish_kernel<<<(int)cgrid, 256, 0, stream>>>(a);
-    if ((rc = launched(1, "pool_finish_kernel launch"))) return rc;
+    if ((rc = launch_pool_centre(a, false, stream))) return rc;
     a.range = scratch + ORDER_RANGE + 2;
     a.queue = refill ? scratch + ORDER_QUEUE2 : nullptr;
     a.queue_ng = nullptr;
     grid = 0;
-    if (refill && (rc = refill_grid(general_variant, a.n, &grid))) return rc;
+    if (refill && (rc = refill_grid(general_variant, a.n, 0, &grid))) return rc;
     return launch_nbody_nodes(a, general_variant, grid, stream);
+}
+
+int launch_nodes_wide(NBodyArgs a, int general_variant, cudaStream_t stream) {
+    a.order = nullptr;
+    a.range = nullptr;
+    a.queue = a.queue_ng = nullptr;
+    int rc = launch_pool(a, NODES_WIDE, (int)a.n, stream);
+    if (rc) return rc;
+    a.pending = 1;
+    return launch_nbody_nodes(a, general_variant, 0, stream);
 }
 
 int preload_nodes_kernels() {
     cudaFuncAttributes fa;
     int rc = 0;
-    for (int v = 0; v <= 10; ++v) {
+    for (int v = 0; v <= NODES_WIDE; ++v)
         if ((rc = cuda_check(cudaFuncGetAttributes(&fa, nodes_kernel_ptr(v)), "load node kernels")))
             return rc;
-        if ((rc = allow_dyn_smem(v))) return rc;
-    }
-    for (const void* f : {(const void*)pool_prepare_kernel, (const void*)pool_finish_kernel})
-        if ((rc = cuda_check(cudaFuncGetAttributes(&fa, f), "load node kernels"))) return rc;
-    return 0;
+    return preload_pool_kernels();
 }
 
 // Resident grid for the persistent (refill) form: blocks per SM from the occupancy API.
-int nodes_grid_size(int variant, int* grid) {
+int nodes_grid_size(int variant, int slots, int* grid) {
     int dev = 0, sms = 0, per_sm = 0;
     int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc) return rc;
     if ((rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")))
         return rc;
-    if ((rc = allow_dyn_smem(variant))) return rc;
+    int smem = 0;
+    if (variant >= 9 && (rc = pool_smem(variant, slots, &smem))) return rc;
     if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                             &per_sm, nodes_kernel_ptr(variant), NODES_BLOCK, dyn_smem(variant)),
+                             &per_sm, nodes_kernel_ptr(variant), NODES_BLOCK, smem),
                          "occupancy")))
         return rc;
     *grid = sms * (per_sm > 0 ? per_sm : 1);

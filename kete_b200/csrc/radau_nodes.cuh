@@ -155,6 +155,7 @@ __global__ void __launch_bounds__(NODES_BLOCK, MINB) nbody_nodes_kernel(NBodyArg
             return false;
         }
         obj = a.order ? a.order[k] : k;
+        if (a.pending && a.status[obj] != ST_PENDING) return false;  // one object per group
         const int64_t n = a.n;
         t = a.jd0[obj];
         tf = a.jd1[obj];
