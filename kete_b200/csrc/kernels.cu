@@ -41,7 +41,7 @@ int upload_ephem(const EphemConst& e) {
 // two-body (kete_core/propagation/kepler.rs:306-322 with the light-delay second pass of the
 // PyO3 binding, src/kete/rust/kepler.rs:89-102).  One thread per object, SoA FP64.
 // -------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) two_body_kernel(
+__global__ void __launch_bounds__(128, 6) two_body_kernel(
     int64_t n, const double* __restrict__ pos, const double* __restrict__ vel,
     const double* __restrict__ jd0, const double* __restrict__ jd1,
     const double* __restrict__ obs, double* __restrict__ out_pos, double* __restrict__ out_vel,
@@ -708,26 +708,58 @@ namespace kb {
 // out (rows x rows) = Phi (rows x cols) C (cols x cols) Phi^T for object i; SoA with the
 // object index fastest.
 __device__ __forceinline__ void covariance_sandwich(int64_t n, int64_t i, int rows, int cols,
-                                                    const double* Phi, bool phi_soa,
-                                                    const double* C, double* out) {
+                                                    const double* Phi, const double* C,
+                                                    double* out) {
     for (int r = 0; r < rows; ++r)
         for (int q = r; q < rows; ++q) {
             double acc = 0.0;
             for (int a = 0; a < cols; ++a) {
-                const double pra = phi_soa ? Phi[(int64_t)(r * cols + a) * n + i] : Phi[r * cols + a];
                 double inner = 0.0;
-                for (int b = 0; b < cols; ++b) {
-                    const double pqb = phi_soa ? Phi[(int64_t)(q * cols + b) * n + i] : Phi[q * cols + b];
-                    inner += C[(int64_t)(a * cols + b) * n + i] * pqb;
-                }
-                acc += pra * inner;
+                for (int b = 0; b < cols; ++b)
+                    inner += C[(int64_t)(a * cols + b) * n + i] * Phi[(int64_t)(q * cols + b) * n + i];
+                acc += Phi[(int64_t)(r * cols + a) * n + i] * inner;
             }
             out[(int64_t)(r * rows + q) * n + i] = acc;
             out[(int64_t)(q * rows + r) * n + i] = acc;
         }
 }
 
-__global__ void __launch_bounds__(128) two_body_stm_kernel(
+// The same for the 6x6 case with Phi in registers: every row of C is read once, the 21 distinct
+// sums grow row by row.
+__device__ __forceinline__ void covariance_sandwich6(int64_t n, int64_t i, const double Phi[36],
+                                                     const double* __restrict__ C,
+                                                     double* __restrict__ out) {
+    double acc[21];
+#pragma unroll
+    for (int k = 0; k < 21; ++k) acc[k] = 0.0;
+#pragma unroll
+    for (int a = 0; a < 6; ++a) {
+        double row[6], inner[6];
+#pragma unroll
+        for (int b = 0; b < 6; ++b) row[b] = __ldg(C + (int64_t)(6 * a + b) * n + i);
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            inner[q] = 0.0;
+#pragma unroll
+            for (int b = 0; b < 6; ++b) inner[q] += row[b] * Phi[6 * q + b];
+        }
+        int k = 0;
+#pragma unroll
+        for (int r = 0; r < 6; ++r)
+#pragma unroll
+            for (int q = r; q < 6; ++q) acc[k++] += Phi[6 * r + a] * inner[q];
+    }
+    int k = 0;
+#pragma unroll
+    for (int r = 0; r < 6; ++r)
+#pragma unroll
+        for (int q = r; q < 6; ++q, ++k) {
+            out[(int64_t)(6 * r + q) * n + i] = acc[k];
+            if (q != r) out[(int64_t)(6 * q + r) * n + i] = acc[k];
+        }
+}
+
+__global__ void __launch_bounds__(128, 3) two_body_stm_kernel(
     int64_t n, const double* __restrict__ pos, const double* __restrict__ vel,
     const double* __restrict__ jd0, const double* __restrict__ jd1, double mu,
     const double* __restrict__ cov, double* __restrict__ out_pos, double* __restrict__ out_vel,
@@ -737,7 +769,25 @@ __global__ void __launch_bounds__(128) two_body_stm_kernel(
     double p[3] = {pos[i], pos[n + i], pos[2 * n + i]};
     double v[3] = {vel[i], vel[n + i], vel[2 * n + i]};
     double Phi[36];
-    int rc = analytic_2_body_stm(jd1[i] - jd0[i], p, v, mu, Phi);
+    // analytic_2_body with its matrix: the whole interval at once, then halves
+    const double time = jd1[i] - jd0[i];
+    int rc = ST_OK;
+    if (fabs(time) < 1e-10) {
+#pragma unroll
+        for (int k = 0; k < 36; ++k) Phi[k] = (k % 7 == 0) ? 1.0 : 0.0;
+    } else if (!two_body_state_ok(p, v)) {
+        rc = ST_CONVERGENCE;
+    } else if (two_body_leaf_stm(time, p, v, mu, Phi) != ST_OK) {
+        double p2[3] = {p[0], p[1], p[2]}, v2[3] = {v[0], v[1], v[2]}, M[36];
+        rc = analytic_2_body_stm_halved(time, p2, v2, mu, M);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            p[c] = p2[c];
+            v[c] = v2[c];
+        }
+#pragma unroll
+        for (int k = 0; k < 36; ++k) Phi[k] = M[k];
+    }
     if (rc != ST_OK) {
         const double nan = __longlong_as_double(0x7ff8000000000000LL);
         p[0] = p[1] = p[2] = v[0] = v[1] = v[2] = nan;
@@ -752,7 +802,7 @@ __global__ void __launch_bounds__(128) two_body_stm_kernel(
     if (out_stm)
 #pragma unroll
         for (int k = 0; k < 36; ++k) out_stm[k * n + i] = Phi[k];
-    if (cov && out_cov) covariance_sandwich(n, i, 6, 6, Phi, false, cov, out_cov);
+    if (cov && out_cov) covariance_sandwich6(n, i, Phi, cov, out_cov);
     status[i] = rc;
 }
 
@@ -762,7 +812,7 @@ __global__ void __launch_bounds__(128) covariance_kernel(int64_t n, int rows, in
                                                          double* __restrict__ out) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    covariance_sandwich(n, i, rows, cols, phi, true, cov, out);
+    covariance_sandwich(n, i, rows, cols, phi, cov, out);
 }
 
 int launch_two_body_stm(int64_t n, const double* pos, const double* vel, const double* jd0,
