@@ -1274,9 +1274,11 @@ static int thermal_model(int model, int64_t n, const double* sun2obj, const doub
         // black_body_flux's per-band constants (common.rs:139-154); bands below 10 nm
         // give no thermal flux
         const double wl_um = band_wavelength[b] * 1e-3;
-        a.bb_k[b] = 1.43877688e4 / wl_um;
+        a.bb_k[b] = band_wavelength[b] < 10.0 ? 1.0 : 1.43877688e4 / wl_um;
         a.bb_coef[b] = band_wavelength[b] < 10.0 ? 0.0 : 397.289171e17 / ((wl_um * wl_um) * wl_um);
     }
+    for (int b = n_bands; b < MAX_BANDS; ++b) a.bb_k[b] = 1.0;
+    for (int b = 0; b < MAX_BANDS; ++b) a.bb_ksum += a.bb_k[b];
     a.have_zero_mags = zero_mags ? 1 : 0;
     a.wise_cc = wise_color_correction ? 1 : 0;
     a.facets = ds->facets;

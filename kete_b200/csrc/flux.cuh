@@ -78,27 +78,6 @@ __device__ __forceinline__ double hg_apparent_flux(const double s2obj[3], const 
     return correction * object_flux_total / (sc2obj_r_km * sc2obj_r_km);
 }
 
-__device__ __forceinline__ double wise_color_correction(int band, double temp) {
-    const double t = clampd(temp, 100.0, 400.0);
-    const double t2 = t * t, t3 = t * t2, t4 = t2 * t2;
-    switch (band) {
-        case 0:
-            return 1.0 / (-3.78226591e-01 + 3.50431748e-03 * t + 1.45866307e-05 * t2 -
-                          6.67674083e-08 * t3 + 7.03651986e-11 * t4);
-        case 1:
-            return 1.0 / (-8.60229377e-01 + 1.54988562e-02 * t - 5.10705456e-05 * t2 +
-                          7.68314436e-08 * t3 - 4.32238900e-11 * t4);
-        case 2:
-            return 1.0 / (-1.29814355 + 2.43268763e-02 * t - 9.05178737e-05 * t2 +
-                          1.50095351e-07 * t3 - 9.35433316e-11 * t4);
-        default: {
-            const double l = log(t), l2 = l * l;
-            return 2.17247804e+01 + -1.46084733e+01 * l + 3.85364000e+00 * l2 -
-                   4.51512551e-01 * (l * l2) + 1.98397252e-02 * (l2 * l2);
-        }
-    }
-}
-
 struct NeatmArgs {
     int model;  // 0 NEATM (neatm.rs), 1 FRM (frm.rs: beaming pi, latitude-only temperatures)
     int64_t n;
@@ -115,7 +94,9 @@ struct NeatmArgs {
     double sun_correction[MAX_BANDS];
     double zero_mag[MAX_BANDS];
     double bb_k[MAX_BANDS];     // black body: exponent numerator 1.43877688e4 / wavelength_um
-    double bb_coef[MAX_BANDS];  // 397.289171e17 / wavelength_um^3; 0 when wavelength < 10 nm
+    double bb_coef[MAX_BANDS];  // 397.289171e17 / wavelength_um^3; 0 when wavelength < 10 nm and
+                                // for the bands beyond n_bands (their bb_k is 1)
+    double bb_ksum;             // sum of bb_k over all MAX_BANDS
     int have_zero_mags;
     int wise_cc;
     const double* band_albedo;  // n_bands x n

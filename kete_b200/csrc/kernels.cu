@@ -482,57 +482,170 @@ int launch_hg_mag(int64_t n, const double* s2obj, const double* s2obs, const dou
 // -------------------------------------------------------------------------------------------
 constexpr int THERMAL_WARPS = 4;
 
+// 1 / x of a normal x, and 1 / sqrt(x) of a normal x > 0, from the hardware's seeds (good to
+// about 20 bits) by one third-order step: with e = 1 - x y, 1 / x = y (1 + e + e^2 + O(e^3)),
+// and with e = 1 - x y^2, 1 / sqrt(x) = y (1 + e / 2 + 3 e^2 / 8 + O(e^3)).
+__device__ __forceinline__ double recip3(double x) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt3(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x * y, y, 1.0);
+    return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+
+// Constants of the facet arithmetic, as constant-bank operands: written as literals the compiler
+// loads them into registers in every batch, two instructions each.
+struct FacetConst {
+    double log2e32, magic, ln2_hi, ln2_lo;  // 32 / ln 2, 1.5 x 2^52, ln 2 / 32 in two parts
+    double e[5];                            // 1/6! .. 1/2!
+    double artanh[10];                      // 1/21, 1/19 .. 1/3
+    double ln2;
+    double w1[5], w2[5], w3[5], w4[5];      // WISE corrections, highest power last
+};
+static __constant__ FacetConst c_fc = {
+    46.16624130844683, 6755399441055744.0, 0x1.62e42fee00000p-6, 0x1.a39ef35793c76p-38,
+    {1.0 / 720.0, 1.0 / 120.0, 1.0 / 24.0, 1.0 / 6.0, 0.5},
+    {1.0 / 21.0, 1.0 / 19.0, 1.0 / 17.0, 1.0 / 15.0, 1.0 / 13.0, 1.0 / 11.0, 1.0 / 9.0, 1.0 / 7.0,
+     1.0 / 5.0, 1.0 / 3.0},
+    0.6931471805599453,
+    {-3.78226591e-01, 3.50431748e-03, 1.45866307e-05, -6.67674083e-08, 7.03651986e-11},
+    {-8.60229377e-01, 1.54988562e-02, -5.10705456e-05, 7.68314436e-08, -4.32238900e-11},
+    {-1.29814355, 2.43268763e-02, -9.05178737e-05, 1.50095351e-07, -9.35433316e-11},
+    {2.17247804e+01, -1.46084733e+01, 3.85364000e+00, -4.51512551e-01, 1.98397252e-02}};
+
+// exp(x) for 0 <= x < 700: x = (32 n + j) ln 2 / 32 + r with ln 2 in two parts (Cody and Waite;
+// the first has 32 significant bits, so its multiples are exact), the exponential's series to
+// r^6 (the next term lies below 4e-18 for |r| <= ln 2 / 64), 2^(j/32) from the block's table,
+// scaled by 2^n.
+constexpr int EXP_TABLE = 32;
+__device__ __forceinline__ double exp_positive(double x, const double* __restrict__ table) {
+    const double t = fma(x, c_fc.log2e32, c_fc.magic);  // the low word is rint(32 x / ln 2)
+    const double n = t - c_fc.magic;
+    const int k = __double2loint(t);
+    double r = fma(-n, c_fc.ln2_hi, x);
+    r = fma(-n, c_fc.ln2_lo, r);
+    double p = c_fc.e[0];
+#pragma unroll
+    for (int i = 1; i < 5; ++i) p = fma(p, r, c_fc.e[i]);
+    p = fma(p * r, r, r);  // exp(r) - 1
+    const double w = table[k & (EXP_TABLE - 1)];
+    const double y = fma(w, p, w);
+    return __hiloint2double(__double2hiint(y) + ((k >> 5) << 20), __double2loint(y));
+}
+
+// log(t) for 100 <= t <= 400: t = 2^e m with m in [2^-1/2, 2^1/2), log m = 2 artanh(s) with
+// s = (m - 1) / (m + 1), |s| <= 0.1716, its series to s^21 (the next term lies below 3e-18).
+__device__ __forceinline__ double log_kelvin(double t) {
+    const int hi = __double2hiint(t);
+    const int e = (hi - 0x3fe6a09e) >> 20;  // t / 2^e in [sqrt(1/2), sqrt(2))
+    const double m = __hiloint2double(hi - (e << 20), __double2loint(t));
+    const double s = (m - 1.0) * recip3(m + 1.0), z = s * s;
+    double p = c_fc.artanh[0];
+#pragma unroll
+    for (int k = 1; k < 10; ++k) p = fma(p, z, c_fc.artanh[k]);
+    const double l = fma(2.0 * s * z, p, 2.0 * s);
+    return fma((double)e, c_fc.ln2, l);
+}
+
+// The WISE colour corrections at temperature t in [100, 400] (constants/wise.rs:40-85): the
+// first three divide, the fourth, of l = log(t), multiplies.
+__device__ __forceinline__ void wise_factors(double t, double l, double& d0, double& d1, double& d2,
+                                             double& w4) {
+    const double t2 = t * t, t3 = t * t2, t4 = t2 * t2, l2 = l * l;
+    const FacetConst& C = c_fc;
+    w4 = C.w4[0] + C.w4[1] * l + C.w4[2] * l2 + C.w4[3] * (l * l2) + C.w4[4] * (l2 * l2);
+    d0 = C.w1[0] + C.w1[1] * t + C.w1[2] * t2 + C.w1[3] * t3 + C.w1[4] * t4;
+    d1 = C.w2[0] + C.w2[1] * t + C.w2[2] * t2 + C.w2[3] * t3 + C.w2[4] * t4;
+    d2 = C.w3[0] + C.w3[1] * t + C.w3[2] * t2 + C.w3[3] * t3 + C.w3[4] * t4;
+}
+
 // Black-body sum of one surviving facet into th[]: temperature from the cos term, then per
 // band coef / (exp(k / T) - 1) (common.rs:139-154) with the WISE colour correction folded
-// into the same division (constants/wise.rs:40-85).
+// into the same division.  Bands the caller does not have carry coef = 0, k = 1.
+//
+// Bound by instruction issue and the FP64 pipe (60% and 55% busy; 11,300 warp instructions a
+// geometry, 21,300 with the library's functions and all of a geometry in one warp; 100,000
+// geometries with four WISE bands 2.27 -> 1.44 ms, with two NEOS bands 1.24 -> 0.80): T = Tss cos^(1/4) and 1 / T
+// come from two reciprocal square roots, the bands' divisions from one reciprocal of their
+// product.  That holds while the exponentials' product stays below e^600 (the WISE and NEOS
+// bands at 30 K: e^311); facets colder than that for their bands take the plain form.
 template <int NB, bool CC>
-__device__ __forceinline__ void thermal_facet(const NeatmArgs& a, double tmp, double seen,
-                                              double ss_temp, double (&th)[NB]) {
-    const double temp = sqrt(sqrt(tmp)) * ss_temp;
-    if (!(temp >= 30.0)) return;
-    const double inv_t = 1.0 / temp;
-    double t = 0.0, t2 = 0.0, t3 = 0.0, t4 = 0.0, w4 = 0.0;
+static __device__ __noinline__ void thermal_facet_cold(const NeatmArgs& a, double temp, double seen,
+                                                       double (&th)[NB]) {
+    double d[3], w4;
     if (CC) {
-        t = clampd(temp, 100.0, 400.0);
-        t2 = t * t;
-        t3 = t * t2;
-        t4 = t2 * t2;
-        const double l = log(t), l2 = l * l;
-        w4 = 2.17247804e+01 + -1.46084733e+01 * l + 3.85364000e+00 * l2 -
-             4.51512551e-01 * (l * l2) + 1.98397252e-02 * (l2 * l2);
+        const double t = clampd(temp, 100.0, 400.0);
+        wise_factors(t, log(t), d[0], d[1], d[2], w4);
     }
-#pragma unroll
     for (int b = 0; b < NB; ++b) {
-        if (b >= a.n_bands || a.bb_coef[b] == 0.0) continue;
-        const double em1 = exp(a.bb_k[b] * inv_t) - 1.0;
-        double ff;
-        if (CC && b == 0)
-            ff = a.bb_coef[b] / (em1 * (-3.78226591e-01 + 3.50431748e-03 * t + 1.45866307e-05 * t2 -
-                                        6.67674083e-08 * t3 + 7.03651986e-11 * t4));
-        else if (CC && b == 1)
-            ff = a.bb_coef[b] / (em1 * (-8.60229377e-01 + 1.54988562e-02 * t - 5.10705456e-05 * t2 +
-                                        7.68314436e-08 * t3 - 4.32238900e-11 * t4));
-        else if (CC && b == 2)
-            ff = a.bb_coef[b] / (em1 * (-1.29814355 + 2.43268763e-02 * t - 9.05178737e-05 * t2 +
-                                        1.50095351e-07 * t3 - 9.35433316e-11 * t4));
-        else if (CC)
-            ff = a.bb_coef[b] / em1 * w4;
-        else
-            ff = a.bb_coef[b] / em1;
-        th[b] += seen * ff;
+        const double em1 = exp(a.bb_k[b] / temp) - 1.0;
+        const double ff = a.bb_coef[b] / (CC && b < 3 ? em1 * d[b < 3 ? b : 0] : em1);
+        th[b] += seen * (CC && b == 3 ? ff * w4 : ff);
     }
 }
 
 template <int NB, bool CC>
-__global__ void __launch_bounds__(32 * THERMAL_WARPS, 8) thermal_kernel(NeatmArgs a) {
-    __shared__ double2 queue[THERMAL_WARPS][64];
+__device__ __forceinline__ void thermal_facet(const NeatmArgs& a, double tmp, double seen,
+                                              double ss_temp, double inv_ss,
+                                              const double* __restrict__ table, double (&th)[NB]) {
+    const double root = tmp * rsqrt3(tmp), w = rsqrt3(root);  // tmp^(1/2), tmp^(-1/4)
+    const double temp = root * w * ss_temp;
+    if (!(temp >= 30.0)) return;
+    const double inv_t = w * inv_ss;
+    if (!(a.bb_ksum * inv_t < 600.0)) {
+        thermal_facet_cold<NB, CC>(a, temp, seen, th);
+        return;
+    }
+    double den[NB];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) den[b] = exp_positive(a.bb_k[b] * inv_t, table) - 1.0;
+    double w4 = 1.0;
+    if (CC) {
+        const double t = clampd(temp, 100.0, 400.0);
+        double d0, d1, d2;
+        wise_factors(t, log_kelvin(t), d0, d1, d2, w4);
+        den[0] *= d0;
+        den[1] *= d1;
+        den[2] *= d2;
+    }
+    // seen / (product of all), then each band's by the product of the others
+    double pre[NB];
+    pre[0] = den[0];
+#pragma unroll
+    for (int b = 1; b < NB; ++b) pre[b] = pre[b - 1] * den[b];
+    double r = seen * recip3(pre[NB - 1]);
+#pragma unroll
+    for (int b = NB - 1; b >= 0; --b) {
+        const double inv = b ? r * pre[b ? b - 1 : 0] : r;
+        r *= den[b];
+        const double ff = a.bb_coef[b] * inv;
+        th[b] = CC && b == 3 ? fma(ff, w4, th[b]) : th[b] + ff;
+    }
+}
+
+// A block takes per_block geometries (a power of two up to THERMAL_MAX): what each needs before
+// the facets and the reflected light after them run one geometry (and band) a thread, the facet
+// sums one geometry a warp.  (With all of it one geometry a warp, the trigonometry of four lanes
+// cost a sixth of the instructions.)
+constexpr int THERMAL_MAX = 16;
+template <int NB, bool CC>
+__global__ void __launch_bounds__(32 * THERMAL_WARPS, 8) thermal_kernel(NeatmArgs a, int per_block) {
+    __shared__ double2 queue[THERMAL_WARPS][96];
+    __shared__ double s_geo[10][THERMAL_MAX];  // to the Sun, to the observer, T, 1 / T, cos, sin
+    __shared__ double s_th[NB][THERMAL_MAX];
+    __shared__ double s_exp[EXP_TABLE];  // 2^(j / 32)
+    if (threadIdx.x < EXP_TABLE) s_exp[threadIdx.x] = exp2(threadIdx.x * (1.0 / EXP_TABLE));
     const int lane = threadIdx.x & 31;
-    double2* q = queue[threadIdx.x >> 5];
-    const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (i >= a.n) return;  // warp-uniform
-    const int64_t n = a.n;
-    double ss_temp, o2s[3], o2o[3], cs = 0.0, sn = 0.0;
-    {
+    const int64_t n = a.n, first = (int64_t)blockIdx.x * per_block;
+    const int count_geo = (int)(n - first < per_block ? n - first : per_block);
+    if ((int)threadIdx.x < count_geo) {
+        const int g = threadIdx.x;
+        const int64_t i = first + g;
         const double s2obj[3] = {a.sun2obj[i], a.sun2obj[n + i], a.sun2obj[2 * n + i]};
         const double s2obs[3] = {a.sun2obs[i], a.sun2obs[n + i], a.sun2obs[2 * n + i]};
         const double obj2sun[3] = {-s2obj[0], -s2obj[1], -s2obj[2]};
@@ -545,105 +658,116 @@ __global__ void __launch_bounds__(32 * THERMAL_WARPS, 8) thermal_kernel(NeatmArg
         const double r2 = obj2sun[0] * obj2sun[0] + obj2sun[1] * obj2sun[1] + obj2sun[2] * obj2sun[2];
         const double reflected = (1.0 - bond_albedo) * SOLAR_FLUX / r2;
         const double beam = a.model == 1 ? PI : a.beaming[i];
-        ss_temp = reflected / (beam * emis * STEFAN_BOLTZMANN);
+        double ss_temp = reflected / (beam * emis * STEFAN_BOLTZMANN);
         ss_temp = ss_temp <= 0.0 ? 0.0 : sqrt(sqrt(ss_temp));
         const double ns = norm3(obj2sun[0], obj2sun[1], obj2sun[2]);
         for (int c = 0; c < 3; ++c) {
-            o2s[c] = obj2sun[c] / ns;
-            o2o[c] = obs2obj[c] / obs2obj_r;
+            s_geo[c][g] = obj2sun[c] / ns;
+            s_geo[3 + c][g] = obs2obj[c] / obs2obj_r;
         }
+        s_geo[6][g] = ss_temp;
+        s_geo[7][g] = 1.0 / ss_temp;  // used where the temperature is at least 30 K
         // FRM: cos(lat_facet - lat_sun) (frm_facet_temperature, frm.rs:19-30) expanded with
         // the facet's cos/sin of latitude from the table
         if (a.model == 1) {
-            const double sun_lat = asin(o2s[2]);
-            cs = cos(sun_lat);
-            sn = sin(sun_lat);
+            const double sun_lat = asin(obj2sun[2] / ns);
+            s_geo[8][g] = cos(sun_lat);
+            s_geo[9][g] = sin(sun_lat);
         }
     }
-    double th[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b) th[b] = 0.0;
+    __syncthreads();
+    double2* q = queue[threadIdx.x >> 5];
     const unsigned below = (1u << lane) - 1u;
-    int count = 0;  // queued facets, warp-uniform
-    for (int base = 0; base < N_FACETS; base += 32) {
-        const int f = base + lane;
-        const double nx = __ldg(a.facets + f), ny = __ldg(a.facets + N_FACETS + f),
-                     nz = __ldg(a.facets + 2 * N_FACETS + f);
-        const double seen = -(nx * o2o[0] + ny * o2o[1] + nz * o2o[2]);
-        double tmp = 0.0;
-        if (seen > 0.0)
-            tmp = a.model == 1 ? __ldg(a.facets + 3 * N_FACETS + f) * cs +
-                                     __ldg(a.facets + 4 * N_FACETS + f) * sn
-                               : nx * o2s[0] + ny * o2s[1] + nz * o2s[2];
-        const bool keep = seen > 0.0 && tmp > 0.0;
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) q[count + __popc(m & below)] = make_double2(tmp, seen);
-        count += __popc(m);
-        if (count >= 32) {
+    const double *t0 = a.facets + (a.model == 1 ? 3 * N_FACETS : 0), *t1 = t0 + N_FACETS;
+    for (int g = threadIdx.x >> 5; g < count_geo; g += THERMAL_WARPS) {
+        const double o0 = s_geo[3][g], o1 = s_geo[4][g], o2 = s_geo[5][g];
+        const double ss_temp = s_geo[6][g], inv_ss = s_geo[7][g];
+        // the temperature's cosine: a table row pair by (c0, c1) plus, NEATM, nz by c2
+        const double c0 = s_geo[a.model == 1 ? 8 : 0][g], c1 = s_geo[a.model == 1 ? 9 : 1][g];
+        const double c2 = a.model == 1 ? 0.0 : s_geo[2][g];
+        double th[NB];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) th[b] = 0.0;
+        int count = 0;  // queued facets, warp-uniform
+        for (int base = 0; base < N_FACETS; base += 64) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int f = base + 32 * half + lane;
+                const double nx = __ldg(a.facets + f), ny = __ldg(a.facets + N_FACETS + f),
+                             nz = __ldg(a.facets + 2 * N_FACETS + f);
+                const double seen = -(nx * o0 + ny * o1 + nz * o2);
+                const double tmp = a.model == 1 ? __ldg(t0 + f) * c0 + __ldg(t1 + f) * c1
+                                                : nx * c0 + ny * c1 + nz * c2;
+                const bool keep = seen > 0.0 && tmp > 0.0;
+                const unsigned m = __ballot_sync(0xffffffffu, keep);
+                if (keep) q[count + __popc(m & below)] = make_double2(tmp, seen);
+                count += __popc(m);
+            }
             __syncwarp();
-            const double2 e = q[lane];
-            thermal_facet<NB, CC>(a, e.x, e.y, ss_temp, th);
+            while (count >= 32) {  // the queue's last 32
+                count -= 32;
+                const double2 e = q[count + lane];
+                thermal_facet<NB, CC>(a, e.x, e.y, ss_temp, inv_ss, s_exp, th);
+            }
             __syncwarp();
-            if (lane < count - 32) q[lane] = q[lane + 32];
-            __syncwarp();
-            count -= 32;
         }
-    }
-    __syncwarp();
-    if (lane < count) {
-        const double2 e = q[lane];
-        thermal_facet<NB, CC>(a, e.x, e.y, ss_temp, th);
-    }
-    // the geometry again, from memory rather than held in registers through the loop
-    const double s2obj[3] = {a.sun2obj[i], a.sun2obj[n + i], a.sun2obj[2 * n + i]};
-    const double s2obs[3] = {a.sun2obs[i], a.sun2obs[n + i], a.sun2obs[2 * n + i]};
-    const double g = a.g_param[i], diam = a.diam[i];
-    // Lambertian scale emissivity * pi * (r / D)^-2 (common.rs:190-205) and the facet area
-    const double obs2obj_r = norm3(s2obj[0] - s2obs[0], s2obj[1] - s2obs[1], s2obj[2] - s2obs[2]);
-    const double dscale = obs2obj_r * AU_KM / diam;
-    const double sc = a.emissivity[i] * PI * (1.0 / (dscale * dscale)) * a.facet_area;
+        if (lane < count) {
+            const double2 e = q[lane];
+            thermal_facet<NB, CC>(a, e.x, e.y, ss_temp, inv_ss, s_exp, th);
+        }
 #pragma unroll
-    for (int b = 0; b < NB; ++b) {
+        for (int b = 0; b < NB; ++b) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) th[b] += __shfl_xor_sync(0xffffffffu, th[b], o);
-        th[b] *= sc;
+            for (int o = 16; o > 0; o >>= 1) th[b] += __shfl_xor_sync(0xffffffffu, th[b], o);
+            if (lane == 0) s_th[b][g] = th[b];
+        }
+        __syncwarp();
     }
-    if (lane < a.n_bands) {
-        const int b = lane;
-        double thb = 0.0;
-#pragma unroll
-        for (int c = 0; c < NB; ++c)
-            if (c == b) thb = th[c];
-        const double refl =
-            hg_apparent_flux(s2obj, s2obs, g, diam, a.wavelength[b], a.band_albedo[(int64_t)b * n + i]) *
-            a.sun_correction[b];
+    __syncthreads();
+    for (int k = threadIdx.x; k < per_block * a.n_bands; k += blockDim.x) {
+        const int b = k / per_block, g = k - b * per_block;
+        if (g >= count_geo) continue;
+        const int64_t i = first + g;
+        const double s2obj[3] = {a.sun2obj[i], a.sun2obj[n + i], a.sun2obj[2 * n + i]};
+        const double s2obs[3] = {a.sun2obs[i], a.sun2obs[n + i], a.sun2obs[2 * n + i]};
+        const double gp = a.g_param[i], diam = a.diam[i];
+        // Lambertian scale emissivity * pi * (r / D)^-2 (common.rs:190-205) and the facet area
+        const double obs2obj_r = norm3(s2obj[0] - s2obs[0], s2obj[1] - s2obs[1], s2obj[2] - s2obs[2]);
+        const double dscale = obs2obj_r * AU_KM / diam;
+        const double thb =
+            s_th[b][g] * (a.emissivity[i] * PI * (1.0 / (dscale * dscale)) * a.facet_area);
+        const double refl = hg_apparent_flux(s2obj, s2obs, gp, diam, a.wavelength[b],
+                                             a.band_albedo[(int64_t)b * n + i]) *
+                            a.sun_correction[b];
         const double total = thb + refl;
         a.thermal[(int64_t)b * n + i] = thb;
         a.hg_fluxes[(int64_t)b * n + i] = refl;
         a.fluxes[(int64_t)b * n + i] = total;
         if (a.mags) a.mags[(int64_t)b * n + i] = a.have_zero_mags ? -2.5 * log10(total / a.zero_mag[b])
                                                                   : __longlong_as_double(0x7ff8000000000000LL);
-    }
-    if (lane == 0) {
-        const double vm = hg_apparent_mag(s2obj, s2obs, a.h_mag[i], g);
-        a.v_mag[i] = vm;
-        a.v_flux[i] = -2.5 * log10(vm / V_MAG_ZERO);  // flux_to_mag(v_mag, V_MAG_ZERO), neatm.rs:167
+        if (b == 0) {
+            const double vm = hg_apparent_mag(s2obj, s2obs, a.h_mag[i], gp);
+            a.v_mag[i] = vm;
+            a.v_flux[i] = -2.5 * log10(vm / V_MAG_ZERO);  // flux_to_mag(v_mag, V_MAG_ZERO), neatm.rs:167
+        }
     }
 }
 
 int launch_neatm(const NeatmArgs& a, cudaStream_t stream) {
     if (a.n <= 0) return 0;
-    const int64_t threads = a.n * 32;
-    const unsigned grid = (unsigned)((threads + 32 * THERMAL_WARPS - 1) / (32 * THERMAL_WARPS));
+    // a warp per geometry until the GPU is full of them, then up to THERMAL_MAX a block
+    int per_block = THERMAL_WARPS;
+    while (per_block < THERMAL_MAX && a.n >= (int64_t)per_block * 148 * 8 * 2) per_block *= 2;
+    const unsigned grid = (unsigned)((a.n + per_block - 1) / per_block);
     const unsigned block = 32 * THERMAL_WARPS;
     if (a.wise_cc)  // the capi admits colour corrections only with the 4 WISE bands
-        thermal_kernel<4, true><<<grid, block, 0, stream>>>(a);
+        thermal_kernel<4, true><<<grid, block, 0, stream>>>(a, per_block);
     else if (a.n_bands <= 2)
-        thermal_kernel<2, false><<<grid, block, 0, stream>>>(a);
+        thermal_kernel<2, false><<<grid, block, 0, stream>>>(a, per_block);
     else if (a.n_bands <= 4)
-        thermal_kernel<4, false><<<grid, block, 0, stream>>>(a);
+        thermal_kernel<4, false><<<grid, block, 0, stream>>>(a, per_block);
     else
-        thermal_kernel<MAX_BANDS, false><<<grid, block, 0, stream>>>(a);
+        thermal_kernel<MAX_BANDS, false><<<grid, block, 0, stream>>>(a, per_block);
     return launched(1, "thermal_kernel launch");
 }
 
