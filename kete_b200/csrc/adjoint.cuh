@@ -465,16 +465,14 @@ struct SensReplayPolicy {
     }
 };
 
-// Jacobian of the force at one point (dual numbers): J (3 x 6) = d a / d(x, v) and
-// jp (3 x 2) = d a / d(A1, A2).  Out of line: one copy serves every call site.
-static __device__ __noinline__ int sens_jacobian(TangentForce& T, double t, const double* x,
-                                          const double* v, double* J, double* jp, EphCache& C) {
+// Jacobian of the force at one point: J (3 x 6) = d a / d(x, v) and jp (3 x 2) = d a / d(A1, A2),
+// in closed form inside the fast plan's window, by dual numbers outside it.  Out of line: one
+// copy serves every call site.
+static __device__ __noinline__ int sens_jacobian_dual(TangentForce& T, double t, const double* x,
+                                                      const double* v, double* J, double* jp) {
     double xx[3] = {x[0], x[1], x[2]}, vv[3] = {v[0], v[1], v[2]};
     double ev[3], JJ[3][6], jj[3][2];
-    const FastPlan& plan = T.n_force == c_eph.n_force_planets ? c_eph.fast_planets : c_eph.fast_all;
-    const int rc = (C.on && t >= plan.lo && t <= plan.hi)
-                       ? T.eval_cached(plan, C, t, xx, vv, ev, JJ, jj)
-                       : T.eval(false, t, xx, vv, ev, JJ, jj);
+    const int rc = T.eval(false, t, xx, vv, ev, JJ, jj);
 #pragma unroll
     for (int r = 0; r < 3; ++r) {
 #pragma unroll
@@ -483,6 +481,19 @@ static __device__ __noinline__ int sens_jacobian(TangentForce& T, double t, cons
         jp[2 * r + 1] = jj[r][1];
     }
     return rc;
+}
+static __device__ __noinline__ int sens_jacobian(TangentForce& T, double t, const double* x,
+                                          const double* v, double* J, double* jp, EphCache& C) {
+    const FastPlan& plan = T.n_force == c_eph.n_force_planets ? c_eph.fast_planets : c_eph.fast_all;
+    if (!(C.on && t >= plan.lo && t <= plan.hi)) return sens_jacobian_dual(T, t, x, v, J, jp);
+    const double xx[3] = {x[0], x[1], x[2]}, vv[3] = {v[0], v[1], v[2]};
+    double JJ[18], jj[6];
+    T.jacobian_cached(plan, C, t, xx, vv, JJ, jj);
+#pragma unroll
+    for (int i = 0; i < 18; ++i) J[i] = JJ[i];
+#pragma unroll
+    for (int i = 0; i < 6; ++i) jp[i] = jj[i];
+    return ST_OK;
 }
 
 // Re-run checkpoint block `c` (its segment ends at tf) with the step code, recording every

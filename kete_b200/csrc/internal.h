@@ -41,6 +41,7 @@ int upload_consts_kernels(const Tables* t, const EphemConst* e);
 int upload_consts_nodes(const Tables* t, const EphemConst* e);
 int upload_consts_pool(const Tables* t, const EphemConst* e);
 int upload_consts_sens(const Tables* t, const EphemConst* e);
+int upload_consts_sens_nodes(const Tables* t, const EphemConst* e);
 int upload_consts_adjoint(const Tables* t, const EphemConst* e);
 int upload_consts_long(const Tables* t, const EphemConst* e);
 
@@ -171,6 +172,7 @@ struct StmArgs {
 };
 // form: 0 = node-parallel (8 lanes per object), 1 = one object per thread
 int launch_nbody_stm(const StmArgs& a, int form, cudaStream_t stream);
+int launch_nbody_stm_thread(const StmArgs& a, cudaStream_t stream);  // sens.cu
 
 // reverse-mode gradients: checkpointed forward pass and adjoint pass (adjoint.cuh)
 constexpr int SENS_STRIDE = 36;       // doubles per checkpoint / attempt record

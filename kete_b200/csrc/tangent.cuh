@@ -247,46 +247,146 @@ struct TangentForce {
         return ST_OK;
     }
 
-    // The same (exact = false) from the fast plan's body positions in the lane's cache,
-    // evaluated at t if the cache holds another time: the bodies are summed in the fast
-    // plan's order (Sun, Jupiter, then the reference's order), a rounding-level change.
-    __device__ int eval_cached(const FastPlan& P, EphCache& C, double t, const double x[3],
-                               const double v[3], double out[3], double J[3][6],
-                               double jp[3][2]) {
+    // The Jacobian alone, in closed form, from the fast plan's body positions in the lane's cache
+    // (evaluated at t if the cache holds another time): what eval's dual numbers give, to
+    // rounding.  Dual numbers carry six derivatives through every operation, and each power of
+    // the comet model's g(r) takes two; here a body costs its 3 x 3 gravity gradient, and the
+    // comet model three powers.
+    __device__ void jacobian_cached(const FastPlan& P, EphCache& C, double t, const double x[3],
+                                    const double v[3], double J[18], double jp[6]) {
         if (t != C.t) {
             SpkForce::fast_positions(P, t, C.p, C.stride);
             C.t = t;
         }
-        D6 acc[3] = {dconst(0.0), dconst(0.0), dconst(0.0)};
-        double dpar[3][2] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-        const double zero[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int i = 0; i < 18; ++i) J[i] = 0.0;
+#pragma unroll
+        for (int i = 0; i < 6; ++i) jp[i] = 0.0;
+        double xx = 0.0, xy = 0.0, xz = 0.0, yy = 0.0, yz = 0.0, zz = 0.0;  // Newtonian part
         const int s = C.stride;
         int k = 0;
+#pragma unroll 1
         for (int it = 0; it < P.n_items; ++it) {
             const FastItem& I = P.item[it];
             if (it >= P.n_vel && I.role < 0) continue;
-            const double bp[3] = {C.p[k * s], C.p[(k + 1) * s], C.p[(k + 2) * s]};
-            double bv[3] = {0.0, 0.0, 0.0};
-            if (it < P.n_vel) {
-                bv[0] = C.p[(k + 3) * s];
-                bv[1] = C.p[(k + 4) * s];
-                bv[2] = C.p[(k + 5) * s];
-                k += 6;
-            } else {
-                k += 3;
+            const double rp[3] = {x[0] - C.p[k * s], x[1] - C.p[(k + 1) * s], x[2] - C.p[(k + 2) * s]};
+            const double ir = rsqrt(rp[0] * rp[0] + rp[1] * rp[1] + rp[2] * rp[2]);
+            const double ir2 = ir * ir, mass = I.mass;
+            const double kk = mass * ir2 * ir, k3 = 3.0 * kk * ir2;
+            // d(-kk r) = -kk I + 3 kk / r^2 r r^T
+            xx += k3 * rp[0] * rp[0] - kk;
+            yy += k3 * rp[1] * rp[1] - kk;
+            zz += k3 * rp[2] * rp[2] - kk;
+            xy += k3 * rp[0] * rp[1];
+            xz += k3 * rp[0] * rp[2];
+            yz += k3 * rp[1] * rp[2];
+            const bool vel = I.kind == FK_SUN || I.kind == FK_JUPITER;
+            if (vel || I.kind == FK_EARTH) {
+                const double q = 1.5 * (I.kind == FK_SUN       ? SUN_J2
+                                        : I.kind == FK_JUPITER ? JUPITER_J2
+                                                               : EARTH_J2) * mass * I.radius * I.radius;
+                const double n[3] = {0.0, vel ? -c_tab.rot_s : 0.0, vel ? c_tab.rot_c : 1.0};
+                j2_gradient(rp, ir, ir2, q, n, J);
             }
-            const ForceEntry fe{I.mass, I.radius, 0, I.kind, I.naif_id, 0};
-            body_dual(fe, ng, x, v, bp, it < P.n_vel ? bv : zero, acc, dpar);
+            if (vel) {
+                const double rv[3] = {v[0] - C.p[(k + 3) * s], v[1] - C.p[(k + 4) * s],
+                                      v[2] - C.p[(k + 5) * s]};
+                gr_gradient(rp, rv, ir, ir2, mass, J);
+                if (I.kind == FK_SUN && ng.kind != 0) nongrav_gradient(ng, rp, rv, ir, J, jp);
+            }
+            k += it < P.n_vel ? 6 : 3;
         }
+        J[0] += xx; J[1] += xy; J[2] += xz;
+        J[6] += xy; J[7] += yy; J[8] += yz;
+        J[12] += xz; J[13] += yz; J[14] += zz;
+    }
+
+    // J2 about the pole n: a = q / r^5 (A r - 2 z n), z = n.r, A = 5 z^2 / r^2 - 1
+    __device__ __forceinline__ static void j2_gradient(const double rp[3], double ir, double ir2,
+                                                       double q, const double n[3], double J[18]) {
+        const double z = n[0] * rp[0] + n[1] * rp[1] + n[2] * rp[2];
+        const double q5 = q * ir2 * ir2 * ir, z2 = z * z * ir2;
+        const double A = 5.0 * z2 - 1.0;
+        const double an = 10.0 * z * ir2, ar = -10.0 * z2 * ir2;  // dA = an n + ar r
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            out[i] = acc[i].v;
+            const double w = -5.0 * q5 * ir2 * (A * rp[i] - 2.0 * z * n[i]);
 #pragma unroll
-            for (int j = 0; j < 6; ++j) J[i][j] = acc[i].d[j];
-            jp[i][0] = dpar[i][0];
-            jp[i][1] = dpar[i][1];
+            for (int c = 0; c < 3; ++c)
+                J[6 * i + c] += q5 * ((i == c ? A : 0.0) + rp[i] * (an * n[c] + ar * rp[c]) -
+                                      2.0 * n[i] * n[c]) + w * rp[c];
         }
-        return ST_OK;
+    }
+
+    // the relativistic term a = g (c r + s v): g = mu / c^2 / r^3, c = 4 mu / r - v^2, s = 4 r.v
+    __device__ __forceinline__ static void gr_gradient(const double rp[3], const double rv[3],
+                                                       double ir, double ir2, double mass,
+                                                       double J[18]) {
+        const double g = mass * C_AU_PER_DAY_INV_SQUARED * ir2 * ir;
+        const double s = 4.0 * (rp[0] * rv[0] + rp[1] * rv[1] + rp[2] * rv[2]);
+        const double c = 4. * mass * ir - (rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2]);
+        const double cr = -4.0 * mass * ir2 * ir;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const double w = -3.0 * ir2 * (c * rp[i] + s * rv[i]) + cr * rp[i];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                J[6 * i + q] += g * ((i == q ? c : 0.0) + 4.0 * rv[i] * rv[q] + w * rp[q]);
+                J[6 * i + 3 + q] += g * ((i == q ? s : 0.0) - 2.0 * rp[i] * rv[q] + 4.0 * rv[i] * rp[q]);
+            }
+        }
+    }
+
+    // Non-gravitational models relative to the Sun.  JPL comet: g(r) (A1 p + A2 t + A3 n) on the
+    // orthonormal frame p = r / |r|, t along the transverse velocity, n = t x p, whose
+    // derivatives stay in the frame:
+    //   dp = (t (t.dr) + n (n.dr)) / r,   dt = n (n.dv - u n.dr) / w - p (t.dr) / r,
+    //   dn = -t (n.dv - u n.dr) / w - p (n.dr) / r,   u = (p.v) / r, w the transverse speed
+    __device__ static void nongrav_gradient(const NonGrav& ng, const double rp[3],
+                                            const double rv[3], double ir, double J[18],
+                                            double jp[6]) {
+        const double p[3] = {rp[0] * ir, rp[1] * ir, rp[2] * ir};
+        const double vr = p[0] * rv[0] + p[1] * rv[1] + p[2] * rv[2];
+        const double w[3] = {rv[0] - p[0] * vr, rv[1] - p[1] * vr, rv[2] - p[2] * vr};
+        if (ng.kind == 2) {  // dust: S ((1 - k v_r) p - k v), S = GM beta / r^2, k = 1 / c^2
+            const double S = GMS * ng.p(1) * ir * ir, kc = C_AU_PER_DAY_INV_SQUARED;
+            const double e = 1.0 - vr * kc;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double D = e * p[i] - kc * rv[i];
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const double id = i == q ? 1.0 : 0.0;
+                    J[6 * i + q] += S * ir * (e * (id - p[i] * p[q]) - 2.0 * D * p[q] - kc * p[i] * w[q]);
+                    J[6 * i + 3 + q] -= S * kc * (p[i] * p[q] + id);
+                }
+            }
+            return;
+        }
+        const double a1 = ng.p(1), a2 = ng.p(2), a3 = ng.p(3), alpha = ng.p(4), r_0 = ng.p(5);
+        const double m = ng.p(6), nn = ng.p(7), kx = ng.p(8);
+        const double iw = rsqrt(w[0] * w[0] + w[1] * w[1] + w[2] * w[2]);
+        const double tv[3] = {w[0] * iw, w[1] * iw, w[2] * iw};
+        const double nv[3] = {tv[1] * p[2] - tv[2] * p[1], tv[2] * p[0] - tv[0] * p[2],
+                              tv[0] * p[1] - tv[1] * p[0]};
+        // g(r) = alpha y^-m (1 + y^n)^-k, y = r / r0; r g' / g = -m - k n y^n / (1 + y^n)
+        const double y = 1.0 / (ir * r_0), yn = pow(y, nn);
+        const double g = alpha * pow(y, -m) * pow(1.0 + yn, -kx);
+        const double gp = g * (-m - kx * nn * yn / (1.0 + yn)) * ir;
+        const double u = vr * ir, gi = g * ir, gw = g * iw;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            jp[2 * i] = p[i] * g;
+            jp[2 * i + 1] = tv[i] * g;
+            const double d = a1 * p[i] + a2 * tv[i] + a3 * nv[i];
+            const double on = gw * (a2 * nv[i] - a3 * tv[i]);  // by n.dv - u n.dr
+            const double ct = gi * (a1 * tv[i] - a2 * p[i]), cn = gi * (a1 * nv[i] - a3 * p[i]);
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                J[6 * i + q] += gp * d * p[q] + ct * tv[q] + (cn - u * on) * nv[q];
+                J[6 * i + 3 + q] += on * nv[q];
+            }
+        }
     }
 };
 
