@@ -122,7 +122,7 @@ __device__ __forceinline__ double3 nongrav_terms(const NonGrav ng, const double3
     const double n_vec[3] = {nv[0] / nnrm, nv[1] / nnrm, nv[2] / nnrm};
     if (DT && dt != 0.0) {
         double p2[3] = {pos[0], pos[1], pos[2]}, v2[3] = {vel[0], vel[1], vel[2]};
-        if (analytic_2_body(-dt, p2, v2) == ST_OK) {
+        if (analytic_2_body_reference(-dt, p2, v2) == ST_OK) {
             pos[0] = p2[0];
             pos[1] = p2[1];
             pos[2] = p2[2];

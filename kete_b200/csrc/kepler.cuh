@@ -53,8 +53,8 @@ struct KepEq {
 // newton_raphson (fitting/newton.rs:18-65): two damped half steps per iteration,
 // the second reusing f unless |f'| < 1e-3.  At most 100 iterations.  One evaluation of the
 // functions at x serves f and f'; g1, g2: at the solution.
-static __device__ __noinline__ int newton(const KepEq& q, double start, double atol, double& out,
-                                          double& g1, double& g2) {
+__device__ __forceinline__ int newton_steps(const KepEq& q, double start, double atol, double& out,
+                                            double& g1, double& g2) {
     double x = start;
     KepEq::At k = q.at(x);
     if (fabs(q.d(k)) < 1e-12) {
@@ -80,6 +80,11 @@ static __device__ __noinline__ int newton(const KepEq& q, double start, double a
         k = q.at(x);
     }
     return ST_CONVERGENCE;
+}
+
+static __device__ __noinline__ int newton(const KepEq& q, double start, double atol, double& out,
+                                          double& g1, double& g2) {
+    return newton_steps(q, start, atol, out, g1, g2);
 }
 
 // The elliptic equation by its true derivatives, all of which one sine and cosine give (with
@@ -157,8 +162,16 @@ struct KeplerStep {
     double s, beta, b_sqrt, g1, g2;
 };
 
+// FAST: kepler_elliptic first.  Without, the reference's iteration alone and inline: fewer
+// registers, for the force kernels that call it around a step loop (the faster form there cost
+// the pooled kernel at 128 registers 156 bytes of spills and 4%).
+template <bool FAST = true>
 __device__ __forceinline__ int solve_kepler_universal(double dt, double r0, double v0, double rv0,
                                                       KeplerStep& o, double mu = GMS) {
+    auto reference = [&](const KepEq& q, double guess) {
+        return FAST ? newton(q, guess, 1e-11, o.s, o.g1, o.g2)
+                    : newton_steps(q, guess, 1e-11, o.s, o.g1, o.g2);
+    };
     const double beta = 2.0 * mu / r0 - powi<2>(v0);
     const double b_sqrt = sqrt(fabs(beta));
     o.beta = beta;
@@ -169,10 +182,10 @@ __device__ __forceinline__ int solve_kepler_universal(double dt, double r0, doub
         const double dtm = fmod_period(dt, period * TAU);
         const KepEq q{r0, rv0, beta, b_sqrt, dtm, false, mu};
         const double guess = (1.0 / b_sqrt) * dtm / period;
-        if (kepler_elliptic(q, guess, 1e-11, o.s, s, c) == ST_OK) {
+        if (FAST && kepler_elliptic(q, guess, 1e-11, o.s, s, c) == ST_OK) {
             o.g1 = 2.0 * s * c / b_sqrt;
             o.g2 = 2.0 * (s * s) / beta;
-        } else if (newton(q, guess, 1e-11, o.s, o.g1, o.g2) != ST_OK) {
+        } else if (reference(q, guess) != ST_OK) {
             return ST_CONVERGENCE;
         }
     } else if (fabs(beta) < PARABOLIC_BETA) {
@@ -189,8 +202,7 @@ __device__ __forceinline__ int solve_kepler_universal(double dt, double r0, doub
         const KepEq q{r0, rv0, beta, b_sqrt, dt, true, mu};
         // kete's starting point uses its GMS_SQRT literal (kepler.rs:228)
         const double mu_sqrt = mu == GMS ? GMS_SQRT : sqrt(mu);
-        if (newton(q, mu_sqrt * fabs(beta) * dt, 1e-11, o.s, o.g1, o.g2) != ST_OK)
-            return ST_CONVERGENCE;
+        if (reference(q, mu_sqrt * fabs(beta) * dt) != ST_OK) return ST_CONVERGENCE;
     }
     return ST_OK;
 }
@@ -215,27 +227,28 @@ __device__ __forceinline__ void two_body_apply(const KeplerStep& k, double r0, d
 }
 
 // One closed-form step; returns ST_CONVERGENCE when the solver fails.
+template <bool FAST = true>
 __device__ __forceinline__ int two_body_leaf(double time, double p[3], double v[3]) {
     const double r0 = norm3(p[0], p[1], p[2]);
     const double v0 = norm3(v[0], v[1], v[2]);
     const double rv0 = p[0] * v[0] + p[1] * v[1] + p[2] * v[2];
     KeplerStep k;
-    if (solve_kepler_universal(time, r0, v0, rv0, k) != ST_OK) return ST_CONVERGENCE;
+    if (solve_kepler_universal<FAST>(time, r0, v0, rv0, k) != ST_OK) return ST_CONVERGENCE;
     two_body_apply(k, r0, rv0, p, v);
     return ST_OK;
 }
 
-// The reference's interval halving (kepler.rs:254-297) once the whole step has failed, in
-// place: a stack of the remaining half-intervals and the depth value their recursive call
-// would receive.  step(dt): one closed-form step of the caller's state; state_ok(): the state is
-// a number.
-template <class Step, class Check>
+// The reference's interval halving (kepler.rs:254-297), in place: a stack of the remaining
+// half-intervals and the depth value their recursive call would receive; WHOLE: from the whole
+// step, otherwise from its halves, once it has failed.  step(dt): one closed-form step of the
+// caller's state; state_ok(): the state is a number.
+template <bool WHOLE, class Step, class Check>
 __device__ __forceinline__ int halved_intervals(double time, Step step, Check state_ok) {
     double st_dt[12];
     int st_depth[12];
-    st_dt[0] = st_dt[1] = time * 0.5;
-    st_depth[0] = st_depth[1] = 1;
-    int top = 2;
+    st_dt[0] = st_dt[1] = WHOLE ? time : time * 0.5;
+    st_depth[0] = st_depth[1] = WHOLE ? 0 : 1;
+    int top = WHOLE ? 1 : 2;
     int guard = 0;
     while (top > 0) {
         if (++guard > 4096) return ST_TIMEOUT;
@@ -262,8 +275,14 @@ __device__ __forceinline__ bool two_body_state_ok(const double p[3], const doubl
 }
 
 static __device__ __noinline__ int analytic_2_body_halved(double time, double p[3], double v[3]) {
-    return halved_intervals(time, [&](double dt) { return two_body_leaf(dt, p, v); },
-                            [&]() { return two_body_state_ok(p, v); });
+    return halved_intervals<false>(time, [&](double dt) { return two_body_leaf(dt, p, v); },
+                                   [&]() { return two_body_state_ok(p, v); });
+}
+
+// The same by the reference's iteration alone (solve_kepler_universal<false>).
+static __device__ __noinline__ int analytic_2_body_reference(double time, double p[3], double v[3]) {
+    return halved_intervals<true>(time, [&](double dt) { return two_body_leaf<false>(dt, p, v); },
+                                  [&]() { return two_body_state_ok(p, v); });
 }
 
 // analytic_2_body (kepler.rs:254-297), in place: the whole interval at once, then halves.

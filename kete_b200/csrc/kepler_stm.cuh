@@ -135,7 +135,7 @@ static __device__ __noinline__ int analytic_2_body_stm_halved(double time, doubl
                                                               double mu, double Phi[36]) {
 #pragma unroll
     for (int k = 0; k < 36; ++k) Phi[k] = (k % 7 == 0) ? 1.0 : 0.0;
-    return halved_intervals(
+    return halved_intervals<false>(
         time,
         [&](double dt) {
             double J[36], tmp[36];
