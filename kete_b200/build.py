@@ -14,8 +14,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libketeb200.so")
 OBJ_DIR = os.path.join(HERE, "_build")  # object files of the incremental build (not shipped)
-SOURCES = ["sens.cu", "sens_nodes.cu", "adjoint.cu", "nodes.cu", "pool.cu", "kernels.cu", "long.cu", "capi.cu",
-           "noalloc.cu"]
+SOURCES = ["sens.cu", "sens_nodes.cu", "sens_pool.cu", "adjoint.cu", "nodes.cu", "pool.cu",
+           "kernels.cu", "long.cu", "capi.cu", "noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -14,8 +14,8 @@ KB_CONSTANT_UPLOADER(adjoint)
 namespace kb {
 
 // Exclusive prefix sums of the blocks each object replays (its checkpoint count when its
-// forward pass succeeded, else none) into a.rep_first[0 .. n], and the replay's queue
-// counter a.rep_first[n + 1] cleared; one thread block, each thread a contiguous run of
+// forward pass succeeded, else none) into a.rep_first[0 .. n], and the replays' queue
+// counters a.rep_first[n + 1], [n + 2] cleared; one thread block, each thread a contiguous run of
 // objects.
 constexpr int OFFSETS_THREADS = 1024;
 __global__ void __launch_bounds__(OFFSETS_THREADS) sens_replay_offsets_kernel(SensArgs a) {
@@ -46,19 +46,27 @@ __global__ void __launch_bounds__(OFFSETS_THREADS) sens_replay_offsets_kernel(Se
     }
     if (threadIdx.x == OFFSETS_THREADS - 1) {
         a.rep_first[n] = (int32_t)s_sum[threadIdx.x];
-        a.rep_first[n + 1] = 0;
+        a.rep_first[n + 1] = a.rep_first[n + 2] = 0;
     }
 }
 
-int launch_sens_forward(const SensArgs& a, cudaStream_t stream) {
-    if (a.n <= 0) return 0;
+int launch_sens_forward(const SensArgs& args, cudaStream_t stream) {
+    if (args.n <= 0) return 0;
+    SensArgs a = args;
+    a.pending = a.pool_slots > 0;
+    if (a.pending) {
+        const int rc = launch_sens_pool_forward(a, stream);
+        if (rc) return rc;
+    }
     const int64_t threads = a.n * SG;
     nbody_sens_forward_kernel<1><<<(unsigned)((threads + SENS_BLOCK - 1) / SENS_BLOCK), SENS_BLOCK, 0, stream>>>(a);
     return launched(1, "nbody_sens_forward_kernel launch");
 }
 
-int launch_sens_backward(const SensArgs& a, cudaStream_t stream) {
-    if (a.n <= 0) return 0;
+int launch_sens_backward(const SensArgs& args, cudaStream_t stream) {
+    if (args.n <= 0) return 0;
+    SensArgs a = args;
+    a.pending = 0;
     const int64_t threads = a.n * SG;
     // the per-lane ephemeris cache takes the block past the 48 KB of shared memory a kernel
     // gets without opting in (a function attribute, not a stream operation)
@@ -86,6 +94,10 @@ int launch_sens_backward(const SensArgs& a, cudaStream_t stream) {
             return rc;
     sens_replay_offsets_kernel<<<1, OFFSETS_THREADS, 0, stream>>>(a);
     if ((rc = launched(1, "sens_replay_offsets_kernel launch"))) return rc;
+    if (a.pool_slots > 0) {
+        if ((rc = launch_sens_pool_replay(a, stream))) return rc;
+        a.pending = 1;
+    }
     // persistent grid: as many thread blocks as are resident at once, and no more than the
     // blocks to replay could occupy
     int dev = 0, sms = 0, per_sm = 0;

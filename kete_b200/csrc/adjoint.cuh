@@ -364,7 +364,7 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_forward_kernel(Se
     const int warp_lane = threadIdx.x & 31;
     const unsigned gmask = 0xFFu << (warp_lane & ~(SG - 1));
     const int64_t obj = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / SG;
-    if (obj >= a.n) return;
+    if (obj >= a.n || (a.pending && a.status[obj] != ST_PENDING)) return;
     double* sb = s_b[threadIdx.x / SG];
     double* se = s_e[threadIdx.x / SG];
     const int comp = lane % 3;
@@ -540,7 +540,7 @@ __device__ __forceinline__ int sens_replay_block(const double* c, double tf, dou
 // a block's replay depends only on its checkpoint, so groups of 8 lanes re-run the blocks in
 // parallel and store each block's attempt records (a.rec_all) and outcome (a.rep_count: the
 // attempt count, or -1 - status on failure) for the sweep to read.  The grid is persistent:
-// each group takes the next block from a queue (a.rep_first[n + 1]) in the dense order of
+// each group takes the next block from a queue (a.rep_first[n + 2]) in the dense order of
 // a.rep_first (sens_replay_offsets_kernel), so groups that finish early take more blocks
 // instead of leaving their thread block's other groups to run alone.
 template <int MINB>
@@ -555,7 +555,7 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(Sen
     const unsigned gmask = 0xFFu << (warp_lane & ~(SG - 1));
     const int64_t n = a.n;
     const int64_t total = a.rep_first[n];
-    int32_t* queue = a.rep_first + n + 1;
+    int32_t* queue = a.rep_first + n + 2;
     double* sb = s_b[threadIdx.x / SG];
     double* se = s_e[threadIdx.x / SG];
     const int comp = lane % 3;
@@ -577,6 +577,7 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(Sen
         const int64_t obj = lo;
         const int cb = (int)(idx - a.rep_first[obj]);
         const int64_t item = obj * a.ckpt_cap + cb;  // the sweep's layout of records and counts
+        if (a.pending && a.rep_count[item] != SENS_PENDING) continue;
         int k = 0;  // the epoch segment holding block cb
         while (k + 1 < a.n_epochs && a.ckpt_seg[(int64_t)(k + 1) * n + obj] <= cb) ++k;
         SpkForce F;

@@ -676,7 +676,8 @@ static int ensure_device(DevState*& out) {
             return rc;
         EphemConst e = g_eph;
         e.pool = ds.pool;
-        if ((rc = upload_ephem(e)) || (rc = upload_pool_plans(g_plans))) return rc;
+        if ((rc = upload_ephem(e)) || (rc = upload_pool_plans(g_plans)) ||
+            (rc = upload_pool_plans_sens(g_plans))) return rc;
         ds.version = g_version;
     }
     out = &ds;
@@ -810,6 +811,12 @@ void nodes_window(int variant, int n_force, double& lo, double& hi) {
 static bool launch_is_default() {
     const LaunchConfig d;
     return g_launch.nodes_variant == d.nodes_variant && g_launch.nodes_refill == d.nodes_refill;
+}
+
+// Doubles of a pooled cache column, 0 where the plan cannot serve.
+static int pool_slots(int n_force) {
+    const PoolPlan& Q = n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
+    return Q.ok ? Q.n_slot : 0;
 }
 
 // What the pooled kernels read besides the plan in constant memory.
@@ -1371,6 +1378,7 @@ int kete_b200_propagate_n_body_stm(int64_t n, const double* pos, const double* v
     a.out_stm = S.out(out_stm, (size_t)n_epochs * 48 * n);
     a.status = S.out(status, (size_t)n);
     a.max_loops = g_launch.max_loops;
+    a.pool_slots = pool_slots(a.n_force);
     if (S.rc) return S.rc;
     if ((rc = launch_nbody_stm(a, g_launch.sens_form, st))) return rc;
     return S.finish();
@@ -1422,6 +1430,7 @@ int kete_b200_propagate_n_body_checkpointed(int64_t n, const double* pos, const 
     a.ckpt_count = S.out(ckpt_count, (size_t)n);
     a.ckpt_seg = S.out(ckpt_segment, (size_t)n_epochs * n);
     a.max_loops = g_launch.max_loops;
+    a.pool_slots = pool_slots(a.n_force);
     if (S.rc) return S.rc;
     if ((rc = launch_sens_forward(a, st))) return rc;
     return S.finish();
@@ -1466,6 +1475,7 @@ int kete_b200_propagate_n_body_adjoint(int64_t n, int n_epochs, const double* ep
     a.out_grad = S.out(out_grad, 8 * (size_t)n);
     a.grad_status = S.out(grad_status, (size_t)n);
     a.max_loops = g_launch.max_loops;
+    a.pool_slots = pool_slots(a.n_force);
     if (S.rc) return S.rc;
     // per-object attempt records of the block being transposed (library scratch)
     void* rec;
@@ -1483,7 +1493,7 @@ int kete_b200_propagate_n_body_adjoint(int64_t n, int n_epochs, const double* ep
         void *ra, *rn, *rf;
         if ((rc = staging(*ds, 35, all_bytes, &ra)) ||
             (rc = staging(*ds, 36, (size_t)n * ckpt_capacity * sizeof(int32_t), &rn)) ||
-            (rc = staging(*ds, 34, ((size_t)n + 2) * sizeof(int32_t), &rf)))
+            (rc = staging(*ds, 34, ((size_t)n + 3) * sizeof(int32_t), &rf)))
             return rc;
         a.rec_all = (double*)ra;
         a.rep_count = (int32_t*)rn;

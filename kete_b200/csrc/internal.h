@@ -42,6 +42,7 @@ int upload_consts_nodes(const Tables* t, const EphemConst* e);
 int upload_consts_pool(const Tables* t, const EphemConst* e);
 int upload_consts_sens(const Tables* t, const EphemConst* e);
 int upload_consts_sens_nodes(const Tables* t, const EphemConst* e);
+int upload_consts_sens_pool(const Tables* t, const EphemConst* e);
 int upload_consts_adjoint(const Tables* t, const EphemConst* e);
 int upload_consts_long(const Tables* t, const EphemConst* e);
 
@@ -169,6 +170,8 @@ struct StmArgs {
     double* out_stm;    // n_epochs x 48 x n (row-major 6 x 8 per object)
     int32_t* status;
     int max_loops;
+    int pool_slots;  // doubles of a pooled cache column, 0: the pooled form cannot serve
+    int pending;     // only the objects whose status is ST_PENDING
 };
 // form: 0 = node-parallel (8 lanes per object), 1 = one object per thread
 int launch_nbody_stm(const StmArgs& a, int form, cudaStream_t stream);
@@ -201,11 +204,18 @@ struct SensArgs {
     double* rec_all;     // n x ckpt_cap x (SENS_CK_ATTEMPTS + 1) x SENS_STRIDE, or null: the
                          // records of every block, replayed up front (adjoint)
     int32_t* rep_count;  // n x ckpt_cap: attempts of each replayed block, -1 - status on failure
-    int32_t* rep_first;  // n + 2 (with rec_all): exclusive prefix sums of the blocks to replay
+    int32_t* rep_first;  // n + 3 (with rec_all): exclusive prefix sums of the blocks to replay
                          // per object (the replay takes the blocks in this dense order), then
-                         // the replay's queue counter
+                         // the queue counters of the pooled and the general replay
     int max_loops;
+    int pool_slots;  // doubles of a pooled cache column, 0: the pooled form cannot serve
+    int pending;     // only the objects whose status is ST_PENDING, the blocks marked SENS_PENDING
 };
+constexpr int SENS_PENDING = -2147483647 - 1;  // rep_count of a block left to the general replay
+// sens_pool.cu: the passes on the warp-pooled step machinery, for what lies inside the window
+int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream);
+int launch_sens_pool_replay(const SensArgs& a, cudaStream_t stream);
+int launch_sens_pool_stm(const StmArgs& a, cudaStream_t stream);
 int launch_sens_forward(const SensArgs& a, cudaStream_t stream);
 int launch_sens_backward(const SensArgs& a, cudaStream_t stream);
 

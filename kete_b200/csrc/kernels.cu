@@ -25,14 +25,16 @@ KB_CONSTANT_UPLOADER(kernels)
 int upload_tables(const Tables& t) {
     int rc = 0;
     for (auto up : {upload_consts_kernels, upload_consts_nodes, upload_consts_pool,
-                    upload_consts_sens, upload_consts_sens_nodes, upload_consts_adjoint, upload_consts_long})
+                    upload_consts_sens, upload_consts_sens_nodes, upload_consts_sens_pool,
+                    upload_consts_adjoint, upload_consts_long})
         if ((rc = up(&t, nullptr))) return rc;
     return 0;
 }
 int upload_ephem(const EphemConst& e) {
     int rc = 0;
     for (auto up : {upload_consts_kernels, upload_consts_nodes, upload_consts_pool,
-                    upload_consts_sens, upload_consts_sens_nodes, upload_consts_adjoint, upload_consts_long})
+                    upload_consts_sens, upload_consts_sens_nodes, upload_consts_sens_pool,
+                    upload_consts_adjoint, upload_consts_long})
         if ((rc = up(nullptr, &e))) return rc;
     return 0;
 }

@@ -32,10 +32,11 @@ struct PoolPlan {
     PoolSeries s[MAX_SERIES];  // n_pos positions (longest first), then velocities
     PoolBody b[MAX_FORCE + 2];
 };
-// The plans of PLANETS and MASSES, in pool.cu's constant memory (upload_pool_plans).
+// The plans of PLANETS and MASSES, in the constant memory of pool.cu and sens_pool.cu.
 struct PoolPlans {
     PoolPlan planets, all;
 };
 int upload_pool_plans(const PoolPlans& p);
+int upload_pool_plans_sens(const PoolPlans& p);
 
 }  // namespace kb

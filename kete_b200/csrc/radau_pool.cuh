@@ -224,12 +224,14 @@ __device__ __forceinline__ void pool_relative(const double x[3], const double* c
 }
 
 // The force at (x, v) from a cache column, one lane summing every body in the plan's order
-// (the non-gravitational term is not included).  Bodies whose positions alone enter go two at
-// a time, their chains interleaved.
+// (the non-gravitational term is not included; NG_SUN: it is na, added after the Sun's terms as
+// the differentiation kernels sum it).  Bodies whose positions alone enter go two at a time,
+// their chains interleaved.
+template <bool NG_SUN = false>
 __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int n_body,
                                             const double* col, int stride, bool exact, bool track,
                                             const double x[3], const double v[3], PoolExact& ex,
-                                            double acc[3]) {
+                                            double acc[3], const double* na = nullptr) {
     acc[0] = acc[1] = acc[2] = 0.0;
 #pragma unroll 1
     for (int i = 0; i < n_vel; ++i) {
@@ -248,6 +250,11 @@ __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int
         acc[0] += t.jm * t.jk;
         acc[1] += t.j1;
         acc[2] += t.j2;
+        if (NG_SUN && i == 0) {
+            acc[0] += na[0];
+            acc[1] += na[1];
+            acc[2] += na[2];
+        }
     }
 #pragma unroll 1
     for (int i = n_vel; i < n_body; i += 2) {
@@ -282,10 +289,12 @@ __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int
 constexpr int TERM_VEL = MAX_FORCE + 2;  // after the kk of every body: 7 a body with velocity
 constexpr int TERM_EARTH = TERM_VEL + 14;
 constexpr int TERM_SLOTS = TERM_EARTH + 2;
+template <bool NG_SUN = false>
 __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_body, int sub,
                                                    const double* col, int stride, double* term,
                                                    bool exact, bool track, const double x[3],
-                                                   const double v[3], PoolExact& ex) {
+                                                   const double v[3], PoolExact& ex,
+                                                   double na = 0.0) {
     const int iv = sub & 1;
     {
         const PoolBody& B = body[iv];
@@ -345,6 +354,7 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
         const double jm = c == 0 ? e[3 * NODE_G] : (c == 1 ? e[5 * NODE_G] : e[6 * NODE_G]);
         const double jk = c == 0 ? e[4 * NODE_G] : 1.0;
         acc += jm * jk;
+        if (NG_SUN && i == 0) acc += na;
     }
     const double coef = term[TERM_EARTH * NODE_G];
     const double z2 = term[(TERM_EARTH + 1) * NODE_G] - (c == 2 ? 3.0 : 1.0);
@@ -485,6 +495,117 @@ struct PoolTables {
     const PoolPlan* plan;
 };
 
+// One round's record evaluations: every series at the times of the groups whose first lane's bit is
+// set in M (TDB seconds in ste, a row of ROWS doubles per group; this group's is gi), into the
+// columns of s_cache.  The 32 lanes take one group's eight columns four lanes each, two groups'
+// two lanes each, or (three or four groups) each lane its own; with S = 4 the warp is one group.
+template <int S, int COLS, int ROWS>
+__device__ __forceinline__ void pool_records(const PoolTables& T, unsigned M, int gi,
+                                             const double* ste, double* s_cache) {
+    const int warp_lane = threadIdx.x & 31, lane = threadIdx.x & (NODE_G - 1);
+    int share, shares, g;
+    if (S > 1) {
+        share = warp_lane / NODE_G;
+        shares = S;
+        g = gi;
+    } else {
+        const unsigned g4 = (M & 1u) | ((M >> 7) & 2u) | ((M >> 14) & 4u) | ((M >> 21) & 8u);
+        const int count = __popc(g4);
+        const int g_lo = __ffs(g4) - 1, g_hi = 31 - __clz(g4);
+        const int own = warp_lane / NODE_G;
+        share = count == 1 ? own : (count == 2 ? (own & 1) : 0);
+        shares = count == 1 ? 4 : (count == 2 ? 2 : 1);
+        g = count == 1 ? g_lo : (count == 2 ? (own < 2 ? g_lo : g_hi) : own);
+        if (count > 2 && !((g4 >> own) & 1u)) share = MAX_SERIES;  // not at new times
+        g += (threadIdx.x >> 5) * (32 / NODE_G);
+    }
+    const double jds = ste[(g - gi) * ROWS + lane];
+    const double* pool = c_eph.pool;
+    double* dst = s_cache + g * NODE_G + lane;
+#pragma unroll 1
+    for (int k = share; k < T.n_pos; k += 3 * shares) {
+        const int kb_ = k + shares, kc = kb_ + shares;
+        const bool has_b = kb_ < T.n_pos, has_c = kc < T.n_pos;
+        pool_positions3<S>(T.src[k], T.src[has_b ? kb_ : k], T.src[has_c ? kc : k], has_b, has_c,
+                           pool, jds, dst, COLS);
+    }
+#pragma unroll 1
+    for (int k = T.n_pos + share; k < T.n_series; k += shares)
+        pool_velocity(T.src[k], pool, jds, dst, COLS);
+    __syncwarp();
+}
+
+// Bodies given relative to a centre (the Earth and Moon), in a node's column after its records.
+__device__ __forceinline__ void pool_chain(const PoolTables& T, double* col, int stride) {
+#pragma unroll 1
+    for (int i = 0; i < T.n_body; ++i) {
+        const int ch = T.plan->b[i].chain, sl = T.plan->b[i].slot;
+        if (ch < 0) continue;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) col[(sl + q) * stride] += col[(ch + q) * stride];
+    }
+}
+
+// The predictor at a node (row nrow) from the group's b and state.
+__device__ __forceinline__ void pool_predict(const double2* nrow, const double* sb,
+                                             const double* st, double xe[3], double ve[3]) {
+    const double2 fr = nrow[8];
+    const double h = st[ST_H], f = fr.x;
+    const double h2 = h * h;
+    const double2* b2 = reinterpret_cast<const double2*>(sb);
+    double bw[3] = {0.0, 0.0, 0.0}, bu[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const double2 w = nrow[k], u = nrow[4 + k];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double2 b = b2[4 * c + k];
+            bw[c] += w.x * b.x;
+            bu[c] += u.x * b.x;
+            if (k < 3) {
+                bw[c] += w.y * b.y;
+                bu[c] += u.y * b.y;
+            }
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double ac = st[ST_A + c], vc = st[ST_V + c];
+        xe[c] = st[ST_X + c] + f * vc * h + fr.y * h2 * (ac / 2.0 + bw[c]);
+        ve[c] = vc + f * h * (ac + bu[c]);
+    }
+}
+
+// One component's corrector: divided differences g of its seven node evaluations (row se),
+// then b = g C into out.
+__device__ __forceinline__ void pool_divided(const double* se, double ac, double g[7], double& e7) {
+    const double2* e2 = reinterpret_cast<const double2*>(se);
+    const double2 e01 = e2[0], e23 = e2[1], e45 = e2[2];
+    const double e[7] = {e01.x, e01.y, e23.x, e23.y, e45.x, e45.y, e2[3].x};
+#pragma unroll
+    for (int j = 1; j < 8; ++j) {
+        double gk = (e[j - 1] - ac) * c_tab.inv_frac[j];
+#pragma unroll
+        for (int z = 1; z < j; ++z) gk = (gk - g[z - 1]) * c_tab.inv_diff[j][z];
+        g[j - 1] = gk;
+    }
+    e7 = e[6];
+}
+__device__ __forceinline__ void pool_store_b(const double g[7], double* out) {
+    double b[8];
+#pragma unroll
+    for (int jj = 0; jj < 7; ++jj) {
+        double s2 = g[jj];
+#pragma unroll
+        for (int k = jj + 1; k < 7; ++k) s2 += c_tab.c[k][jj] * g[k];
+        b[jj] = s2;
+    }
+    b[7] = 0.0;
+    double2* o = reinterpret_cast<double2*>(out);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k] = make_double2(b[2 * k], b[2 * k + 1]);
+}
+
 // PREPARED: objects of the order, from queues (a.queue; S = 4: its heavy objects) or, without,
 // one per group, with pool_prepare_kernel before and pool_finish_kernel after; otherwise one
 // per group in the caller's order, centre and frame changed here.
@@ -515,7 +636,6 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
     const bool se_lane = lane == 7;
     double* col = s_cache + gi * NODE_G + lane;
     const bool track = a.min_dist != nullptr;
-    const double* pool = c_eph.pool;
 
     int64_t obj = -1;
     int phase = PH_DONE;
@@ -691,47 +811,8 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
                 ste[lane] = __dmul_rn(te - 2451545.0, 86400.0);
             }
             __syncwarp();
-            // which column this lane evaluates, and its share of the series: the 32 lanes take
-            // one group's eight columns four lanes each, two groups' two lanes each, or (three
-            // or four groups) each lane its own
-            int share, shares, g;
-            if (S > 1) {
-                share = sub;
-                shares = S;
-                g = gi;
-            } else {
-                const unsigned g4 = (M & 1u) | ((M >> 7) & 2u) | ((M >> 14) & 4u) | ((M >> 21) & 8u);
-                const int count = __popc(g4);
-                const int g_lo = __ffs(g4) - 1, g_hi = 31 - __clz(g4);
-                const int own = warp_lane / NODE_G;
-                share = count == 1 ? own : (count == 2 ? (own & 1) : 0);
-                shares = count == 1 ? 4 : (count == 2 ? 2 : 1);
-                g = count == 1 ? g_lo : (count == 2 ? (own < 2 ? g_lo : g_hi) : own);
-                if (count > 2 && !((g4 >> own) & 1u)) share = MAX_SERIES;  // not at new times
-                g += (threadIdx.x >> 5) * (32 / NODE_G);
-            }
-            const double jds = ste[(g - gi) * Sh::ROWS + lane];
-            double* dst = s_cache + g * NODE_G + lane;
-#pragma unroll 1
-            for (int k = share; k < T.n_pos; k += 3 * shares) {
-                const int kb_ = k + shares, kc = kb_ + shares;
-                const bool has_b = kb_ < T.n_pos, has_c = kc < T.n_pos;
-                pool_positions3<S>(T.src[k], T.src[has_b ? kb_ : k], T.src[has_c ? kc : k], has_b,
-                                   has_c, pool, jds, dst, COLS);
-            }
-#pragma unroll 1
-            for (int k = T.n_pos + share; k < T.n_series; k += shares)
-                pool_velocity(T.src[k], pool, jds, dst, COLS);
-            __syncwarp();
-            if (need && sub == 0) {  // bodies given relative to a centre (the Earth and Moon)
-#pragma unroll 1
-                for (int i = 0; i < T.n_body; ++i) {
-                    const int ch = T.plan->b[i].chain, sl = T.plan->b[i].slot;
-                    if (ch < 0) continue;
-#pragma unroll
-                    for (int q = 0; q < 3; ++q) col[(sl + q) * COLS] += col[(ch + q) * COLS];
-                }
-            }
+            pool_records<S, COLS, Sh::ROWS>(T, M, gi, ste, s_cache);
+            if (need && sub == 0) pool_chain(T, col, COLS);
             if (S > 1) __syncwarp();
             fresh = false;
         }
@@ -744,31 +825,7 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
                 ve[c] = st[ST_V + c];
             }
         } else {
-            const double2 fr = nrow[8];
-            const double h = st[ST_H], f = fr.x;
-            const double h2 = h * h;
-            const double2* b2 = reinterpret_cast<const double2*>(sb);
-            double bw[3] = {0.0, 0.0, 0.0}, bu[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double2 w = nrow[k], u = nrow[4 + k];
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const double2 b = b2[4 * c + k];
-                    bw[c] += w.x * b.x;
-                    bu[c] += u.x * b.x;
-                    if (k < 3) {
-                        bw[c] += w.y * b.y;
-                        bu[c] += u.y * b.y;
-                    }
-                }
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const double ac = st[ST_A + c], vc = st[ST_V + c];
-                xe[c] = st[ST_X + c] + f * vc * h + fr.y * h2 * (ac / 2.0 + bw[c]);
-                ve[c] = vc + f * h * (ac + bu[c]);
-            }
+            pool_predict(nrow, sb, st, xe, ve);
         }
         const bool exact = !iter_round || se_lane;
         PoolExact ex;
@@ -830,38 +887,16 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
         bool conv;
         {
             const double ac = st[ST_A + comp];
-            const double2* e2 = reinterpret_cast<const double2*>(se + NODE_G * comp);
-            const double2 e01 = e2[0], e23 = e2[1], e45 = e2[2];
-            const double e[7] = {e01.x, e01.y, e23.x, e23.y, e45.x, e45.y, e2[3].x};
-            double g[7];
-#pragma unroll
-            for (int j = 1; j < 8; ++j) {
-                double gk = (e[j - 1] - ac) * c_tab.inv_frac[j];
-#pragma unroll
-                for (int z = 1; z < j; ++z) gk = (gk - g[z - 1]) * c_tab.inv_diff[j][z];
-                g[j - 1] = gk;
-            }
+            double g[7], e7;
+            pool_divided(se + NODE_G * comp, ac, g, e7);
             // converged when |b6 - b6_old| / (|a at node 7| + 1e-6) is below 1e-14 in every
             // component, as products; a NaN counts as below while another component is not one
             const double change = fabs(g[6] - sb[POOL_B * comp + 6]);
-            const double limit = 1e-14 * (fabs(e[6]) + 1e-6);
+            const double limit = 1e-14 * (fabs(e7) + 1e-6);
             const unsigned above = __ballot_sync(gmask, owner && change >= limit);
             const unsigned number = __ballot_sync(gmask, owner && change == change);
             conv = above == 0 && number != 0;
-            if (owner) {
-                double b[8];
-#pragma unroll
-                for (int jj = 0; jj < 7; ++jj) {
-                    double s2 = g[jj];
-#pragma unroll
-                    for (int k = jj + 1; k < 7; ++k) s2 += c_tab.c[k][jj] * g[k];
-                    b[jj] = s2;
-                }
-                b[7] = 0.0;
-                double2* o = reinterpret_cast<double2*>(sb + POOL_B * comp);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) o[k] = make_double2(b[2 * k], b[2 * k + 1]);
-            }
+            if (owner) pool_store_b(g, sb + POOL_B * comp);
         }
         __syncwarp(gmask);
         ++iter;
@@ -934,9 +969,9 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
 }
 
 // Fills the block's tables (static shared memory of the kernels).
-__device__ __forceinline__ PoolTables pool_tables(const NBodyArgs& a, double* s_node,
+__device__ __forceinline__ PoolTables pool_tables(int n_force, double* s_node,
                                                   PoolSeries* s_src, PoolBody* s_body) {
-    const PoolPlan& plan = a.n_force == c_eph.n_force_planets ? c_plans.planets : c_plans.all;
+    const PoolPlan& plan = n_force == c_eph.n_force_planets ? c_plans.planets : c_plans.all;
     for (int i = threadIdx.x; i < 9 * POOL_NODE; i += blockDim.x) {
         const int j = i / POOL_NODE, k = i % POOL_NODE;
         double val = 0.0;
@@ -967,7 +1002,7 @@ __global__ void __launch_bounds__(NODES_BLOCK, MINB) nbody_pool_kernel(NBodyArgs
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
     __shared__ PoolSeries s_src[MAX_SERIES];
     __shared__ PoolBody s_body[MAX_FORCE + 2];
-    const PoolTables T = pool_tables(a, s_node, s_src, s_body);
+    const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
     if (HEAVY) {
         if ((int)blockIdx.x * (NODES_BLOCK / 32) < a.wide[0] + a.wide[1])
             pool_run<4, NODES_BLOCK, true>(a, T, s_pool);
@@ -986,7 +1021,7 @@ __global__ void __launch_bounds__(WIDE_BLOCK, MINB) nbody_wide_kernel(NBodyArgs 
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
     __shared__ PoolSeries s_src[MAX_SERIES];
     __shared__ PoolBody s_body[MAX_FORCE + 2];
-    const PoolTables T = pool_tables(a, s_node, s_src, s_body);
+    const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
     pool_run<4, WIDE_BLOCK, false>(a, T, s_pool);
 }
 

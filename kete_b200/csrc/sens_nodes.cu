@@ -12,9 +12,16 @@
 namespace kb {
 KB_CONSTANT_UPLOADER(sens_nodes)
 
-int launch_nbody_stm(const StmArgs& a, int form, cudaStream_t stream) {
-    if (a.n <= 0) return 0;
+int launch_nbody_stm(const StmArgs& args, int form, cudaStream_t stream) {
+    if (args.n <= 0) return 0;
+    StmArgs a = args;
+    a.pending = 0;
     if (form == 1) return launch_nbody_stm_thread(a, stream);
+    if (a.pool_slots > 0) {
+        const int prc = launch_sens_pool_stm(a, stream);
+        if (prc) return prc;
+        a.pending = 1;
+    }
     // node-parallel: tangents in dynamic shared memory above the 48 KB static limit (a
     // function attribute, set on every launch: it is not a stream operation)
     int rc = cuda_check(cudaFuncSetAttribute(nbody_stm_nodes_kernel<1>,

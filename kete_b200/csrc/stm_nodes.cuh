@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(STM_BLOCK, MINB) nbody_stm_nodes_kernel(StmArg
     const int warp_lane = threadIdx.x & 31;
     const unsigned gmask = 0xFFu << (warp_lane & ~(SG - 1));
     const int64_t obj = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / SG;
-    if (obj >= a.n) return;
+    if (obj >= a.n || (a.pending && a.status[obj] != ST_PENDING)) return;
     double* sb = s_b[threadIdx.x / SG];
     double* se = s_e[threadIdx.x / SG];
     double* ts = s_tan + (threadIdx.x / SG) * STM_ROW;
