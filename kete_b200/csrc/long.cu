@@ -15,31 +15,26 @@ int launch_nbody_long(const LongArgs& a, cudaStream_t stream) {
     const int64_t n_batch = (a.n + a.batch - 1) / a.batch;
     const int m = LONG_MASSIVE + a.batch;
     const bool comets = a.nongrav != nullptr;
+    // The points over a block, faster at any number of batches (10 particles, ten years: 200
+    // batches 19.2 ms and 81.5 for a thread per body, with comets 46.2 and 180.6; 1000 batches
+    // 65.4 and 91.9, with comets 181.5 and 206.4).
     if (m <= LP_BODIES) {
-        const int threads = long_points_threads(m), smem = long_points_doubles(m) * (int)sizeof(double);
+        const int threads = long_points_threads(m), smem = long_points_doubles(m, comets) * (int)sizeof(double);
         const bool narrow = threads <= LP_NARROW;
         const auto kernel = narrow ? (comets ? nbody_long_points_kernel<LP_NARROW, 2, true>
                                              : nbody_long_points_kernel<LP_NARROW, 2, false>)
                                    : (comets ? nbody_long_points_kernel<LP_WIDE, 1, true>
                                              : nbody_long_points_kernel<LP_WIDE, 1, false>);
-        int dev = 0, sms = 0, rc;
-        if ((rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice")) ||
-            (rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")) ||
-            (rc = cuda_check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  long_points_doubles(LP_BODIES) * (int)sizeof(double)),
-                             "nbody_long_points_kernel shared memory")))
-            return rc;
-        // Without comets at any number of batches (10 particles, ten years: 200 batches 19.2 ms
-        // and 81.5 for a thread per body, 1000 batches 65.4 and 91.9).  The comet model is a call
-        // whose registers the kernel spills around: while the batches are one wave (200: 58.9
-        // and 180.6), not beyond (1000: 221.6 and 207.5).
-        if (!comets || n_batch <= (int64_t)sms * (narrow ? 2 : 1)) {
-            kernel<<<(unsigned)n_batch, threads, smem, stream>>>(a);
-            return launched(1, "nbody_long_points_kernel launch");
-        }
+        const int rc = cuda_check(
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 long_points_doubles(LP_BODIES, true) * (int)sizeof(double)),
+            "nbody_long_points_kernel shared memory");
+        if (rc) return rc;
+        kernel<<<(unsigned)n_batch, threads, smem, stream>>>(a);
+        return launched(1, "nbody_long_points_kernel launch");
     }
-    const int block = LONG_MASSIVE + a.batch <= 32 ? 32 : 64;
-    nbody_long_kernel<<<(unsigned)n_batch, block, 0, stream>>>(a);
+    // larger batches: a thread per body
+    nbody_long_kernel<<<(unsigned)n_batch, 64, 0, stream>>>(a);
     return launched(1, "nbody_long_kernel launch");
 }
 

@@ -334,18 +334,19 @@ __global__ void __launch_bounds__(64) nbody_long_kernel(LongArgs a) {
 // 200 batches of 10 over ten years (1062 steps, 5574 iterations): 19.2 ms, on 52 of 148 SMs two
 // blocks; 130 batches 13.3 ms, one batch 11.5 ms.  A warp per node whose lanes went through the
 // nine pairs took 28.8 ms (13,900 instructions an iteration against 9,400, 23% of the FP64 pipe).
-// NG: with the comet model, whose call costs the kernel 1.4 KB of spills, kept out of the build
-// without.
+// NG: with the comet model, whose call costs the kernel 1.8 KB of spills, kept out of the build
+// without (46.2 ms; 58.8 with the model's term in the Sun's warps, 50.6 for a warp per node).
 // -------------------------------------------------------------------------------------------
 constexpr int LP_BODIES = 32;
 constexpr int LP_SUBS = 3;
 constexpr int LP_SETS = 4;
 constexpr int LP_NARROW = 480, LP_WIDE = 7 * LP_BODIES * LP_SUBS;  // threads of the two builds
-constexpr int LP_TERMS = 7;  // the first three bodies' sum, then a term each
+constexpr int LP_TERMS = 7;     // the first three bodies' sum, then a term each
+constexpr int LP_NG_TERMS = 3;  // with comets: the third body in its place; the Sun, Mercury, comet
 
 // doubles of shared memory for m bodies: the points' states, terms and accelerations, |b6|
-__host__ __device__ constexpr int long_points_doubles(int m) {
-    return 7 * m * (6 + 3 * LP_TERMS + 3) + 3 * m;
+__host__ __device__ constexpr int long_points_doubles(int m, bool ng) {
+    return 7 * m * (6 + 3 * (LP_TERMS + (ng ? LP_NG_TERMS : 0)) + 3) + 3 * m;
 }
 __host__ __device__ constexpr int long_points_threads(int m) {
     return LP_SUBS * 32 * ((7 * m + 31) / 32);
@@ -388,26 +389,23 @@ __device__ __forceinline__ int long_terms(int sub, const double* X, double* W, i
     };
     if (sub == 0) {
         double s[3];
-        if (NG && ng.kind != 0) {  // first, while little is live, and kept in the term's place
-            const double3 na = nongrav_accel(
-                ng, make_double3(xe[0] - X[p0], xe[1] - X[P + p0], xe[2] - X[2 * P + p0]),
-                make_double3(X[3 * P + p] - X[3 * P + p0], X[4 * P + p] - X[4 * P + p0],
-                             X[5 * P + p] - X[5 * P + p0]));
-            w[0] = na.x;
-            w[1] = na.y;
-            w[2] = na.z;
-            store(0);
-        }
         long_term<0, EXACT>(X, P, p, p0, body, xe, hit, s);
-        if (NG && ng.kind != 0)
+        if (NG) {  // the comet term comes in between
 #pragma unroll
-            for (int c = 0; c < 3; ++c) s[c] += W[c * P + p];
+            for (int c = 0; c < 3; ++c) W[(3 * LP_TERMS + c) * P + p] = s[c];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) s[c] = 0.0;
+        }
         long_term<1, EXACT>(X, P, p, p0, body, xe, hit, w);
+        if (NG) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) W[(3 * LP_TERMS + 3 + c) * P + p] = w[c];
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c) s[c] += w[c];
         long_term<2, EXACT>(X, P, p, p0, body, xe, hit, w);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) w[c] = s[c] + w[c];
+        for (int c = 0; c < 3; ++c) w[c] = NG ? w[c] : s[c] + w[c];
         store(0);
     } else if (sub == 1) {
         long_term<5, EXACT>(X, P, p, p0, body, xe, hit, w);
@@ -417,6 +415,16 @@ __device__ __forceinline__ int long_terms(int sub, const double* X, double* W, i
         long_term<4, EXACT>(X, P, p, p0, body, xe, hit, w);
         store(2);
     } else {
+        if (NG && ng.kind != 0) {
+            const double3 rp = make_double3(xe[0] - X[p0], xe[1] - X[P + p0], xe[2] - X[2 * P + p0]);
+            const double3 rv = make_double3(X[3 * P + p] - X[3 * P + p0], X[4 * P + p] - X[4 * P + p0],
+                                            X[5 * P + p] - X[5 * P + p0]);
+            const double3 na = ng.kind == 1 && ng.p(9) == 0.0 ? nongrav_terms<false>(ng, rp, rv)
+                                                              : nongrav_accel(ng, rp, rv);
+            W[(3 * LP_TERMS + 6) * P + p] = na.x;
+            W[(3 * LP_TERMS + 7) * P + p] = na.y;
+            W[(3 * LP_TERMS + 8) * P + p] = na.z;
+        }
         long_term<6, EXACT>(X, P, p, p0, body, xe, hit, w);
         store(4);
         long_term<7, EXACT>(X, P, p, p0, body, xe, hit, w);
@@ -427,9 +435,15 @@ __device__ __forceinline__ int long_terms(int sub, const double* X, double* W, i
     return hit;
 }
 
-// Component c of the acceleration at point p.
-__device__ __forceinline__ double long_sum(const double* W, int P, int p, int c) {
+// Component c of the acceleration at point p (comet: the point's body has a comet term).
+template <bool NG>
+__device__ __forceinline__ double long_sum(const double* W, int P, int p, int c, bool comet) {
     double acc = W[c * P + p];
+    if (NG) {
+        double w = W[(3 * LP_TERMS + c) * P + p];
+        if (comet) w += W[(3 * LP_TERMS + 6 + c) * P + p];
+        acc = (w + W[(3 * LP_TERMS + 3 + c) * P + p]) + acc;
+    }
 #pragma unroll
     for (int k = 1; k < LP_TERMS; ++k) acc += W[(3 * k + c) * P + p];
     return acc;
@@ -448,7 +462,7 @@ __global__ void __launch_bounds__(THREADS, MINB) nbody_long_points_kernel(LongAr
     const int P = 7 * m, C = 3 * m;
     double* X = s_long;
     double* W = X + 6 * P;
-    double* E = W + 3 * LP_TERMS * P;
+    double* E = W + 3 * (LP_TERMS + (NG ? LP_NG_TERMS : 0)) * P;
     double* s_b6 = E + 3 * P;
     const int t0 = threadIdx.x, warp = t0 >> 5, lane = t0 & 31;
     // this thread's point and share of its terms
@@ -470,7 +484,7 @@ __global__ void __launch_bounds__(THREADS, MINB) nbody_long_points_kernel(LongAr
     ng.base = nullptr;
     ng.stride = n;
     ng.kind = 0;
-    if (NG && point && sub == 0 && body > LONG_MASSIVE) {
+    if (NG && point && body > LONG_MASSIVE) {
         ng.base = a.nongrav + i0 + (body - LONG_MASSIVE);
         ng.kind = (int)*ng.base;
     }
@@ -499,7 +513,7 @@ __global__ void __launch_bounds__(THREADS, MINB) nbody_long_points_kernel(LongAr
         exact_sync();
         if (p < m && long_terms<true, NG>(sub, X, W, P, p, 0, body, ng)) s_hit = 1;
         exact_sync();
-        if (p < m) E[sub * P + p] = long_sum(W, P, p, sub);
+        if (p < m) E[sub * P + p] = long_sum<NG>(W, P, p, sub, ng.kind != 0);
     };
     if (exact_warp) exact();
     __syncthreads();
@@ -538,7 +552,7 @@ __global__ void __launch_bounds__(THREADS, MINB) nbody_long_points_kernel(LongAr
                 __syncthreads();
                 if (point) long_terms<false, NG>(sub, X, W, P, p, p0, body, ng);
                 __syncthreads();
-                if (point) E[sub * P + p] = long_sum(W, P, p, sub);
+                if (point) E[sub * P + p] = long_sum<NG>(W, P, p, sub, ng.kind != 0);
                 __syncthreads();
                 int above = 0;
                 if (task) {

@@ -1,6 +1,5 @@
 """The system integration's forms: batches of up to 23 test particles with their points spread
-over a block (two builds, each with and without the comet model), a thread per body above and,
-with comets, beyond one wave of blocks."""
+over a block (two builds, each with and without the comet model), a thread per body above."""
 import numpy as np
 import pytest
 
@@ -32,8 +31,7 @@ def test_block_edges_vs_oracle(gpu, oracle_spk, batch, n, comets):
 
 
 def test_comets_beyond_a_wave_and_impact(gpu):
-    """301 batches with comets take a thread per body, the first ten alone do not: the same sums
-    in the same order, bit for bit.  A particle inside the Sun ends its batch, and only that."""
+    """301 batches, more than one wave of blocks, and the first ten alone: bit for bit.  A particle inside the Sun ends its batch, and only that."""
     n, batch = 903, 3
     pos, vel, ng = _states(n, 8)
     first = [np.ascontiguousarray(x[:, :30]) for x in (pos, vel, ng)]
