@@ -71,7 +71,9 @@ def init(device: int | None = None):
         try:
             import torch
 
-            device = torch.cuda.current_device() if torch.cuda.is_available() else 0
+            # a set-up context answers without asking for the devices again (1.5 us a call)
+            ready = torch.cuda.is_initialized() or torch.cuda.is_available()
+            device = torch.cuda.current_device() if ready else 0
         except Exception:  # torch absent or no GPU: let the library report it
             device = 0
     if device not in _initialised:
@@ -80,7 +82,7 @@ def init(device: int | None = None):
 
 
 def _is_torch_cuda(a) -> bool:
-    return type(a).__module__.startswith("torch") and getattr(a, "is_cuda", False)
+    return getattr(a, "is_cuda", False) and type(a).__module__.startswith("torch")
 
 
 class Args:
@@ -103,7 +105,8 @@ class Args:
             if self.stream is None:
                 import torch
 
-                self.stream = torch.cuda.current_stream(a.device).cuda_stream
+                # the raw handle: torch.cuda.current_stream wraps it in a Stream (4 us)
+                self.stream = torch._C._cuda_getCurrentRawStream(a.get_device())
             self.keep.append(a)
             return a.data_ptr()
         if self.device is True:
