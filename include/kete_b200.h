@@ -57,6 +57,8 @@ extern "C" {
 #define KETE_B200_FRAME_ECLIPTIC 2
 
 /* propagate_n_body modes */
+/* AUTO: by the object count (a warp per object up to 4,096, the warp-pooled forms above) until
+ * kete_b200_set_launch_config installs a configuration, then that configuration */
 #define KETE_B200_MODE_AUTO 0
 #define KETE_B200_MODE_THREAD 1  /* one object per thread, one launch per call */
 #define KETE_B200_MODE_NODES 2   /* eight lanes per object: the 7 Gauss-Radau nodes in parallel */
@@ -378,8 +380,8 @@ int kete_b200_set_launch_config(int nodes_variant, int nodes_refill, int thread_
 int kete_b200_set_step_limit(int64_t max_steps);
 
 /* Form of the N-body forward sensitivities (kete_b200_propagate_n_body_stm and the N-body
- * covariance propagation built on it; no counterpart in the reference): 0 (default) = eight
- * lanes per object, each corrector node's force Jacobian taken once per step attempt at its
+ * covariance propagation built on it; no counterpart in the reference): 0 (default) = a warp
+ * per object, each corrector node's force Jacobian taken once per step attempt at its
  * last iteration's point; 1 = one object per thread, every iteration's Jacobian at its own
  * points.  The two agree to about 1e-8 relative. */
 int kete_b200_set_sensitivity_form(int form);
@@ -388,7 +390,7 @@ int kete_b200_set_sensitivity_form(int form);
  * reference): 0 (default) = every checkpoint block of every object re-run in one parallel
  * launch before the sweep, when their records fit a bounded library scratch (8 GiB; else as
  * 1); 1 = the sweep re-runs each block itself, just before transposing it.  Both give the same
- * gradients bit for bit. */
+ * gradients bit for bit (with the asteroid masses to rounding). */
 int kete_b200_set_adjoint_form(int form);
 
 /* Form of the field checks (kete_b200_fov_check_visible and the schedule built on it; no

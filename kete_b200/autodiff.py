@@ -47,7 +47,7 @@ def _bind():
 
 
 def set_sensitivity_form(form: int = 0):
-    """Form of the forward sensitivities (kete_b200_set_sensitivity_form): 0 = eight lanes per
+    """Form of the forward sensitivities (kete_b200_set_sensitivity_form): 0 = a warp per
     object with each node's Jacobian taken once per step attempt (default); 1 = one object
     per thread with every corrector iteration's Jacobian at its own points."""
     L = _lib.lib()

@@ -786,8 +786,8 @@ int nodes_variant_for(int variant, int n_force) {
 //   variant 10 209    513    542    664     836    3545   (128 registers, refill)
 // A warp per object is the shortest wait until the warps fill the GPU twice; above, four
 // objects share a warp, and the 128-register form's extra warps pay once the queue holds many
-// objects per lane group (a +-5 yr mix of 125,000: 16.5 ms against 17.8; a million: 125.0
-// against 135.8).
+// objects per lane group (a +-5 yr mix of 125,000: 16.1 ms against 17.8; a million: 121.9
+// against 136.0).
 constexpr int64_t AUTO_WIDE_MAX = 4096, AUTO_168_MAX = 98304;
 static int auto_variant(int64_t n, int n_force) {
     const PoolPlan& Q = n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;

@@ -28,7 +28,7 @@
 // FP64 pipe is 33% active.  Replacing the library's rsqrt and pow by shorter chains, merging
 // the terms of Sun and Jupiter and scaling the coefficients on the host changed nothing
 // (133.5 ms against 132.6 on the million), so the arithmetic stays as it was.  Per warp round
-// the instructions fell from 2730 to 2180; a million objects of the mix take 125 ms (171.3
+// the instructions fell from 2730 to 2180; a million objects of the mix take 122 ms (171.3
 // before, 261 in the form that the library used without tuning), 10,000 of the main belt over a
 // year 0.75 ms (1.0).
 //

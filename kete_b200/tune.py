@@ -11,6 +11,9 @@ evaluations across all 32 lanes) and in two grid forms (one lane group per objec
 persistent grid whose groups take the next object from a queue).  Which is fastest depends on the object
 count and the spread of their step counts, so it is measured: ``autotune`` times every
 configuration on the caller's own inputs (device arrays) and installs the fastest.
+
+Until a configuration is installed, the automatic mode picks by the object count (a warp per
+object up to 4,096, then variants 9 and 10 with the queue); the explicit mode runs variant 7.
 """
 from __future__ import annotations
 

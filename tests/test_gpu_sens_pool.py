@@ -3,8 +3,8 @@
 they leave to the general kernels: started outside the ephemeris, a NaN state, a comet
 with a delay.  States and sensitivities against the one-object-per-thread form, with the
 bounds that it is held to elsewhere (1e-9 AU, 1e-7 of a column); the gradients against the
-transposed sensitivities (1e-8 of a parameter group); the replays bit for bit where the plans
-evaluate the same records."""
+transposed sensitivities (1e-8 of a parameter group); the replays bit for bit where both
+read positions from the cache."""
 import numpy as np
 import pytest
 
@@ -78,7 +78,7 @@ def _check(A, n, asteroids):
     err = (np.abs(m1 - m0).max(axis=1) / np.abs(m0).max(axis=1))[..., ok]
     assert np.nanmax(err) < 1e-7
     assert np.array_equal(np.isnan(m1), np.isnan(m0))
-    if not asteroids:  # their centre, the Sun, is evaluated once here and once more there
+    if not asteroids:  # the general replay takes them without the cache of rounded positions
         assert np.array_equal(g[0], g[1], equal_nan=True)
     ref = np.einsum("kcn,kcpn->pn", seed, m1.reshape(K, 6, 8, n))[:, ok]
     for rows in (slice(0, 3), slice(3, 6)):
