@@ -379,6 +379,13 @@ static void build_pool_plan(const FastPlan& P, PoolPlan& Q) {
         S.slot = Q.b[v].vslot = Q.n_slot;
         Q.n_slot += 3;
     }
+    Q.km = fast_plan_cache_doubles(P) > EPH_CACHE;
+    for (int v = 0; v < Q.n_vel; ++v) {
+        const PoolSeries& S = Q.s[Q.n_pos + v];
+        Q.b[v].vscale = g_pool_host[S.offset + 2];
+        for (int64_t r = 1; r < S.n_rec; ++r)  // unscaled columns need one scale a series
+            if (Q.km && g_pool_host[S.offset + r * S.rsize + 2] != Q.b[v].vscale) return;
+    }
     PoolBody& D = Q.b[Q.n_body];
     D = Q.b[Q.n_body - 1];
     D.mass = D.j2m = 0.0;
@@ -823,6 +830,7 @@ static int pool_slots(int n_force) {
 static void set_pool(NBodyArgs& a, double lo, double hi) {
     const PoolPlan& Q = a.n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
     a.pool_slots = Q.n_slot;
+    a.pool_km = Q.km;
     a.lo = lo;
     a.hi = hi;
 }

@@ -73,6 +73,7 @@ struct NBodyArgs {
     int* wide;            // pooled kernels: {heavy objects leading the order's first part, those
                           // leading its non-gravitational part, the queue of both}
     int pool_slots;       // pooled kernels: doubles of a cache column (PoolPlan::n_slot)
+    int pool_km;          // ... unscaled columns (PoolPlan::km)
     double lo, hi;        // wide pooled kernel: the fast plan's window
     int pending;          // node kernel: only the objects whose status is ST_PENDING
 };

@@ -18,13 +18,19 @@ int upload_pool_plans(const PoolPlans& p) {
     return cuda_check(cudaMemcpyToSymbol(c_plans, &p, sizeof(PoolPlans)), "upload pooled plans");
 }
 
-const void* pool_kernel_ptr(int variant) {
+static const void* kernel_ptr(int variant, bool km) {
     switch (variant) {
-        case NODES_WIDE: return (const void*)nbody_wide_kernel<16>;
-        case 9: return (const void*)nbody_pool_kernel<3, true>;
-        default: return (const void*)nbody_pool_kernel<4, true>;
+        case NODES_WIDE:
+            return km ? (const void*)nbody_wide_kernel<16, true> : (const void*)nbody_wide_kernel<16, false>;
+        case 9:
+            return km ? (const void*)nbody_pool_kernel<3, true, true>
+                      : (const void*)nbody_pool_kernel<3, true, false>;
+        default:
+            return km ? (const void*)nbody_pool_kernel<4, true, true>
+                      : (const void*)nbody_pool_kernel<4, true, false>;
     }
 }
+const void* pool_kernel_ptr(int variant) { return kernel_ptr(variant, false); }
 
 // Dynamic shared memory of a variant for cache columns of `slots` doubles.  Above the 48 KB
 // static limit it has to be allowed once per device (a function attribute, not a stream
@@ -46,11 +52,12 @@ int pool_smem(int variant, int slots, int* bytes) {
     const unsigned long long bit = 1ull << (dev & 63);
     auto& d = done[variant - 9];
     if (d.load() & bit) return 0;
-    if ((rc = cuda_check(cudaFuncSetAttribute(pool_kernel_ptr(variant),
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              pool_bytes(variant, POOL_MAX_SLOTS)),
-                         "pooled kernel shared memory")))
-        return rc;
+    for (bool km : {false, true})
+        if ((rc = cuda_check(cudaFuncSetAttribute(kernel_ptr(variant, km),
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  pool_bytes(variant, POOL_MAX_SLOTS)),
+                             "pooled kernel shared memory")))
+            return rc;
     d.fetch_or(bit);
     return 0;
 }
@@ -59,12 +66,18 @@ int launch_pool(const NBodyArgs& a, int variant, int grid, cudaStream_t stream) 
     int smem = 0;
     const int rc = pool_smem(variant, a.pool_slots, &smem);
     if (rc) return rc;
-    if (variant == NODES_WIDE)
-        nbody_wide_kernel<16><<<grid, WIDE_BLOCK, smem, stream>>>(a);
+    if (variant == NODES_WIDE && a.pool_km)
+        nbody_wide_kernel<16, true><<<grid, WIDE_BLOCK, smem, stream>>>(a);
+    else if (variant == NODES_WIDE)
+        nbody_wide_kernel<16, false><<<grid, WIDE_BLOCK, smem, stream>>>(a);
+    else if (variant == 9 && a.pool_km)
+        nbody_pool_kernel<3, true, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
     else if (variant == 9)
-        nbody_pool_kernel<3, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
+        nbody_pool_kernel<3, true, false><<<grid, NODES_BLOCK, smem, stream>>>(a);
+    else if (a.pool_km)
+        nbody_pool_kernel<4, true, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
     else
-        nbody_pool_kernel<4, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
+        nbody_pool_kernel<4, true, false><<<grid, NODES_BLOCK, smem, stream>>>(a);
     return launched(1, "nbody_pool_kernel launch");
 }
 
@@ -79,7 +92,7 @@ int preload_pool_kernels() {
     cudaFuncAttributes fa;
     int rc = 0, smem = 0;
     for (const void* f : {(const void*)pool_prepare_kernel, (const void*)pool_finish_kernel,
-                          pool_kernel_ptr(NODES_WIDE)})
+                          kernel_ptr(NODES_WIDE, false), kernel_ptr(NODES_WIDE, true)})
         if ((rc = cuda_check(cudaFuncGetAttributes(&fa, f), "load pooled kernels"))) return rc;
     for (int v : {9, 10})
         if ((rc = pool_smem(v, POOL_MAX_SLOTS, &smem))) return rc;

@@ -18,10 +18,10 @@ struct PoolSeries {
 };
 // One body of the pooled force sum, in the fast plan's order (the bodies with velocities, then
 // the others; b[n_body] is a copy of the last one without mass or radius, the partner of an odd
-// one).  j2m: 1.5 J2 mass; chain: cache slot of the centre whose position the body's is
+// one).  j2m: 1.5 J2 mass; vscale: the velocity series' scale; chain: cache slot of the centre whose position the body's is
 // relative to (-1: none).
 struct PoolBody {
-    double mass, radius, radius2, j2m;
+    double mass, radius, radius2, j2m, vscale;
     int32_t slot, vslot, chain, naif_id, kind, pad_;
 };
 constexpr int MAX_SERIES = 24;
@@ -29,6 +29,7 @@ constexpr int POOL_MAX_SLOTS = 57;  // doubles of a cache column (planets 39, wi
 constexpr int POOL_EARTH = 4;  // the Earth's place in the plan: Sun, Jupiter, Mercury, Venus, Earth
 struct PoolPlan {
     int32_t ok, n_pos, n_series, n_body, n_vel, n_slot;
+    int32_t km, pad_;  // 1: unscaled columns (radau_pool.cuh), for a plan too large for EPH_CACHE
     PoolSeries s[MAX_SERIES];  // n_pos positions (longest first), then velocities
     PoolBody b[MAX_FORCE + 2];
 };

@@ -67,7 +67,7 @@ __device__ __forceinline__ const double2* pool_record(const PoolSeries& S, const
 // The positions of three series at one time, in lockstep (nine sums and three recurrences in
 // flight); the second and third may be shorter than the first.  The arithmetic of each is
 // cheb_pos3's.
-template <int S>
+template <int S, bool KM>
 __device__ __forceinline__ void pool_positions3(const PoolSeries& A, const PoolSeries& B,
                                                 const PoolSeries& C, bool has_b, bool has_c,
                                                 const double* __restrict__ pool, double jds,
@@ -116,7 +116,7 @@ __device__ __forceinline__ void pool_positions3(const PoolSeries& A, const PoolS
                 t1[q] = nt;
             }
     }
-    constexpr double INV_AU_KM = 1.0 / AU_KM;
+    constexpr double INV_AU_KM = KM ? 1.0 : 1.0 / AU_KM;
     const int slot[3] = {A.slot, B.slot, C.slot};
 #pragma unroll
     for (int q = 0; q < 3; ++q)
@@ -128,6 +128,7 @@ __device__ __forceinline__ void pool_positions3(const PoolSeries& A, const PoolS
 }
 
 // The velocity of one series (cheb_pair's arithmetic).
+template <bool KM>
 __device__ __forceinline__ void pool_velocity(const PoolSeries& A, const double* __restrict__ pool,
                                               double jds, double* col, int stride) {
     const double2* r = pool_record(A, pool, jds);
@@ -157,7 +158,7 @@ __device__ __forceinline__ void pool_velocity(const PoolSeries& A, const double*
     }
     double* d = col + A.slot * stride;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) d[c * stride] = acc[c] * tss;
+    for (int c = 0; c < 3; ++c) d[c * stride] = KM ? acc[c] : acc[c] * tss;
 }
 
 // What an exact evaluation reports besides the acceleration.
@@ -223,11 +224,35 @@ __device__ __forceinline__ void pool_relative(const double x[3], const double* c
     for (int k = 0; k < 3; ++k) r[k] = x[k] - c[k * stride];
 }
 
+// KM: the columns hold the series' sums unscaled (chained bodies: their positions), and the
+// scaling is fused into the differences, as the general forms evaluate a plan that does not fit
+// their per-lane cache (the asteroid masses): the results are then theirs to the bit but for one
+// object in three hundred.  (Rounded positions differ from theirs in every object, which close
+// approaches took to 9e-8 of the velocities' scale within two years; the time is the same.)
+constexpr double POOL_INV_AU = 1.0 / AU_KM;
+template <bool KM>
+__device__ __forceinline__ void pool_body_position(const PoolBody& B, const double x[3],
+                                                   const double* col, int stride, double r[3]) {
+    const double* c = col + B.slot * stride;
+    if (!KM) return pool_relative(x, c, stride, r);
+    const double scale = B.chain >= 0 ? 1.0 : POOL_INV_AU;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r[k] = fma(-c[k * stride], scale, x[k]);
+}
+template <bool KM>
+__device__ __forceinline__ void pool_body_velocity(const PoolBody& B, const double v[3],
+                                                   const double* col, int stride, double r[3]) {
+    const double* c = col + B.vslot * stride;
+    if (!KM) return pool_relative(v, c, stride, r);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) r[k] = fma(-c[k * stride], B.vscale, v[k]);
+}
+
 // The force at (x, v) from a cache column, one lane summing every body in the plan's order
 // (the non-gravitational term is not included; NG_SUN: it is na, added after the Sun's terms as
 // the differentiation kernels sum it).  Bodies whose positions alone enter go two at a time,
 // their chains interleaved.
-template <bool NG_SUN = false>
+template <bool NG_SUN = false, bool KM = false>
 __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int n_body,
                                             const double* col, int stride, bool exact, bool track,
                                             const double x[3], const double v[3], PoolExact& ex,
@@ -237,8 +262,8 @@ __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int
     for (int i = 0; i < n_vel; ++i) {
         const PoolBody& B = body[i];
         double rp[3], rv[3];
-        pool_relative(x, col + B.slot * stride, stride, rp);
-        pool_relative(v, col + B.vslot * stride, stride, rv);
+        pool_body_position<KM>(B, x, col, stride, rp);
+        pool_body_velocity<KM>(B, v, col, stride, rv);
         const double r2 = pool_r2(rp);
         pool_checks(B, r2, exact, track, ex);
         const PoolVel t = pool_vel_terms(B, rp, rv, r2);
@@ -260,8 +285,8 @@ __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int
     for (int i = n_vel; i < n_body; i += 2) {
         const PoolBody &A = body[i], &B = body[i + 1];
         double ra[3], rb[3];
-        pool_relative(x, col + A.slot * stride, stride, ra);
-        pool_relative(x, col + B.slot * stride, stride, rb);
+        pool_body_position<KM>(A, x, col, stride, ra);
+        pool_body_position<KM>(B, x, col, stride, rb);
         const double r2a = pool_r2(ra), r2b = pool_r2(rb);
         const double ia = rsqrt(r2a), ib = rsqrt(r2b);
         const double ia3 = ia * ia * ia, ib3 = ib * ib * ib;
@@ -289,7 +314,7 @@ __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int
 constexpr int TERM_VEL = MAX_FORCE + 2;  // after the kk of every body: 7 a body with velocity
 constexpr int TERM_EARTH = TERM_VEL + 14;
 constexpr int TERM_SLOTS = TERM_EARTH + 2;
-template <bool NG_SUN = false>
+template <bool NG_SUN = false, bool KM = false>
 __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_body, int sub,
                                                    const double* col, int stride, double* term,
                                                    bool exact, bool track, const double x[3],
@@ -299,8 +324,8 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
     {
         const PoolBody& B = body[iv];
         double rp[3], rv[3];
-        pool_relative(x, col + B.slot * stride, stride, rp);
-        pool_relative(v, col + B.vslot * stride, stride, rv);
+        pool_body_position<KM>(B, x, col, stride, rp);
+        pool_body_velocity<KM>(B, v, col, stride, rv);
         const double r2 = pool_r2(rp);
         if (sub < 2) pool_checks(B, r2, exact, track, ex);
         const PoolVel t = pool_vel_terms(B, rp, rv, r2);
@@ -315,8 +340,8 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
         const int i = min(i0 + 2 * sub, n_body), k = min(i0 + 2 * sub + 1, n_body);
         const PoolBody &A = body[i], &B = body[k];
         double ra[3], rb[3];
-        pool_relative(x, col + A.slot * stride, stride, ra);
-        pool_relative(x, col + B.slot * stride, stride, rb);
+        pool_body_position<KM>(A, x, col, stride, ra);
+        pool_body_position<KM>(B, x, col, stride, rb);
         const double r2a = pool_r2(ra), r2b = pool_r2(rb);
         const double ia = rsqrt(r2a), ib = rsqrt(r2b);
         const double ia3 = ia * ia * ia, ib3 = ib * ib * ib;
@@ -348,7 +373,9 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const double* e = term + (TERM_VEL + 7 * i) * NODE_G;
-        const double rp = xc - cc[body[i].slot * stride], rv = vc - cc[body[i].vslot * stride];
+        const double bp = cc[body[i].slot * stride], bv = cc[body[i].vslot * stride];
+        const double rp = KM ? fma(-bp, POOL_INV_AU, xc) : xc - bp;
+        const double rv = KM ? fma(-bv, body[i].vscale, vc) : vc - bv;
         acc -= rp * term[i * NODE_G];
         acc += e[0] * (e[NODE_G] * rp + e[2 * NODE_G] * rv);
         const double jm = c == 0 ? e[3 * NODE_G] : (c == 1 ? e[5 * NODE_G] : e[6 * NODE_G]);
@@ -360,7 +387,8 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
     const double z2 = term[(TERM_EARTH + 1) * NODE_G] - (c == 2 ? 3.0 : 1.0);
 #pragma unroll 4
     for (int i = 2; i < n_body; ++i) {
-        const double rp = xc - cc[body[i].slot * stride];
+        const double bp = cc[body[i].slot * stride];
+        const double rp = KM ? fma(-bp, body[i].chain >= 0 ? 1.0 : POOL_INV_AU, xc) : xc - bp;
         acc -= rp * term[i * NODE_G];
         if (i == POOL_EARTH) acc += rp * coef * z2;
     }
@@ -499,7 +527,7 @@ struct PoolTables {
 // set in M (TDB seconds in ste, a row of ROWS doubles per group; this group's is gi), into the
 // columns of s_cache.  The 32 lanes take one group's eight columns four lanes each, two groups'
 // two lanes each, or (three or four groups) each lane its own; with S = 4 the warp is one group.
-template <int S, int COLS, int ROWS>
+template <int S, int COLS, int ROWS, bool KM = false>
 __device__ __forceinline__ void pool_records(const PoolTables& T, unsigned M, int gi,
                                              const double* ste, double* s_cache) {
     const int warp_lane = threadIdx.x & 31, lane = threadIdx.x & (NODE_G - 1);
@@ -526,23 +554,28 @@ __device__ __forceinline__ void pool_records(const PoolTables& T, unsigned M, in
     for (int k = share; k < T.n_pos; k += 3 * shares) {
         const int kb_ = k + shares, kc = kb_ + shares;
         const bool has_b = kb_ < T.n_pos, has_c = kc < T.n_pos;
-        pool_positions3<S>(T.src[k], T.src[has_b ? kb_ : k], T.src[has_c ? kc : k], has_b, has_c,
+        pool_positions3<S, KM>(T.src[k], T.src[has_b ? kb_ : k], T.src[has_c ? kc : k], has_b, has_c,
                            pool, jds, dst, COLS);
     }
 #pragma unroll 1
     for (int k = T.n_pos + share; k < T.n_series; k += shares)
-        pool_velocity(T.src[k], pool, jds, dst, COLS);
+        pool_velocity<KM>(T.src[k], pool, jds, dst, COLS);
     __syncwarp();
 }
 
 // Bodies given relative to a centre (the Earth and Moon), in a node's column after its records.
+template <bool KM = false>
 __device__ __forceinline__ void pool_chain(const PoolTables& T, double* col, int stride) {
 #pragma unroll 1
     for (int i = 0; i < T.n_body; ++i) {
         const int ch = T.plan->b[i].chain, sl = T.plan->b[i].slot;
         if (ch < 0) continue;
 #pragma unroll
-        for (int q = 0; q < 3; ++q) col[(sl + q) * stride] += col[(ch + q) * stride];
+        for (int q = 0; q < 3; ++q) {
+            double& p = col[(sl + q) * stride];
+            const double centre = col[(ch + q) * stride];
+            p = KM ? fma(p, POOL_INV_AU, __dmul_rn(centre, POOL_INV_AU)) : p + centre;
+        }
     }
 }
 
@@ -609,7 +642,7 @@ __device__ __forceinline__ void pool_store_b(const double g[7], double* out) {
 // PREPARED: objects of the order, from queues (a.queue; S = 4: its heavy objects) or, without,
 // one per group, with pool_prepare_kernel before and pool_finish_kernel after; otherwise one
 // per group in the caller's order, centre and frame changed here.
-template <int S, int THREADS, bool PREPARED>
+template <int S, int THREADS, bool PREPARED, bool KM>
 __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T, double* smem) {
     using Sh = PoolShared<S, THREADS>;
     constexpr int GL = NODE_G * S, COLS = Sh::COLS;  // lanes of a group; cache columns
@@ -811,8 +844,8 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
                 ste[lane] = __dmul_rn(te - 2451545.0, 86400.0);
             }
             __syncwarp();
-            pool_records<S, COLS, Sh::ROWS>(T, M, gi, ste, s_cache);
-            if (need && sub == 0) pool_chain(T, col, COLS);
+            pool_records<S, COLS, Sh::ROWS, KM>(T, M, gi, ste, s_cache);
+            if (need && sub == 0) pool_chain<KM>(T, col, COLS);
             if (S > 1) __syncwarp();
             fresh = false;
         }
@@ -833,16 +866,17 @@ __device__ __forceinline__ void pool_run(const NBodyArgs& a, const PoolTables& T
         ex.min_r2 = min_r2;
         double ev[3];  // S > 1: ev[0] is the sub-lane's component
         if (S > 1)
-            ev[0] = pool_forces_wide(T.body, T.n_body, sub, col, COLS, term, exact, track, xe, ve, ex);
+            ev[0] = pool_forces_wide<false, KM>(T.body, T.n_body, sub, col, COLS, term, exact, track, xe, ve, ex);
         else
-            pool_forces(T.plan->b, T.n_vel, T.n_body, col, COLS, exact, track, xe, ve, ex, ev);
+            pool_forces<false, KM>(T.plan->b, T.n_vel, T.n_body, col, COLS, exact, track, xe, ve, ex, ev);
         if (ng.kind != 0) {
             // non_grav_accel relative to the Sun (acceleration.rs:161-165): inline for the
             // JPL comet model without delay; a call for the delayed model and dust
-            const double* sc = col + T.plan->b[0].slot * COLS;
-            const double* sv = col + T.plan->b[0].vslot * COLS;
-            const double3 rp = make_double3(xe[0] - sc[0], xe[1] - sc[COLS], xe[2] - sc[2 * COLS]);
-            const double3 rv = make_double3(ve[0] - sv[0], ve[1] - sv[COLS], ve[2] - sv[2 * COLS]);
+            double sx[3], sv[3];
+            pool_body_position<KM>(T.plan->b[0], xe, col, COLS, sx);
+            pool_body_velocity<KM>(T.plan->b[0], ve, col, COLS, sv);
+            const double3 rp = make_double3(sx[0], sx[1], sx[2]);
+            const double3 rv = make_double3(sv[0], sv[1], sv[2]);
             const double3 na = (ng.kind == 1 && ng.p(9) == 0.0) ? nongrav_terms<false>(ng, rp, rv)
                                                                 : nongrav_accel(ng, rp, rv);
             if (S > 1) {
@@ -996,7 +1030,7 @@ __device__ __forceinline__ PoolTables pool_tables(int n_force, double* s_node,
 // others when those are taken.  The objects with many times the steps of most (near the Earth,
 // long spans) bound a launch of a few objects per lane group: see order_scan_kernel for the
 // rule.
-template <int MINB, bool HEAVY>
+template <int MINB, bool HEAVY, bool KM>
 __global__ void __launch_bounds__(NODES_BLOCK, MINB) nbody_pool_kernel(NBodyArgs a) {
     extern __shared__ __align__(16) double s_pool[];
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
@@ -1005,24 +1039,24 @@ __global__ void __launch_bounds__(NODES_BLOCK, MINB) nbody_pool_kernel(NBodyArgs
     const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
     if (HEAVY) {
         if ((int)blockIdx.x * (NODES_BLOCK / 32) < a.wide[0] + a.wide[1])
-            pool_run<4, NODES_BLOCK, true>(a, T, s_pool);
+            pool_run<4, NODES_BLOCK, true, KM>(a, T, s_pool);
         __syncthreads();
     }
-    pool_run<1, NODES_BLOCK, true>(a, T, s_pool);
+    pool_run<1, NODES_BLOCK, true, KM>(a, T, s_pool);
 }
 
 // A warp an object in the caller's order, blocks of one warp so that few objects spread over
 // the SMs; centre and frame are changed here, and the objects whose span leaves the window are
 // left to the general form.
 constexpr int WIDE_BLOCK = 32;
-template <int MINB>
+template <int MINB, bool KM>
 __global__ void __launch_bounds__(WIDE_BLOCK, MINB) nbody_wide_kernel(NBodyArgs a) {
     extern __shared__ __align__(16) double s_pool[];
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
     __shared__ PoolSeries s_src[MAX_SERIES];
     __shared__ PoolBody s_body[MAX_FORCE + 2];
     const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
-    pool_run<4, WIDE_BLOCK, false>(a, T, s_pool);
+    pool_run<4, WIDE_BLOCK, false, KM>(a, T, s_pool);
 }
 
 }  // namespace kb
