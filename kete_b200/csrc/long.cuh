@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(64) nbody_long_kernel(LongArgs a) {
 // evaluation.
 // 200 batches of 10 over ten years (1062 steps, 5574 iterations): 19.2 ms, on 52 of 148 SMs two
 // blocks; 130 batches 13.3 ms, one batch 11.5 ms.  A warp per node whose lanes went through the
-// nine pairs took 28.8 ms (13,900 instructions an iteration against 9,400, 23% of the FP64 pipe).
+// nine pairs took 28.8 ms (13,900 instructions an iteration against 8,500, 23% of the FP64 pipe against 31%).
 // NG: with the comet model, whose call costs the kernel 1.8 KB of spills, kept out of the build
 // without (46.2 ms; 58.8 with the model's term in the Sun's warps, 50.6 for a warp per node).
 // -------------------------------------------------------------------------------------------
