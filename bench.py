@@ -82,8 +82,8 @@ NODE_TRAFFIC = {
     ("nbody_mixed_1m", 7, 1): {"bytes_per_object": (13_601_536 + 882_944) / 100_000,
                                "fp64_pipe": 0.217,
                                "captured": "one launch on a 100,000-object sample of the workload"},
-    ("nbody_mixed_1m", 10, 1): {"bytes_per_object": (12_881_920 + 127_488) / 100_000,
-                                "fp64_pipe": 0.326,
+    ("nbody_mixed_1m", 10, 1): {"bytes_per_object": (12_840_000 + 55_040) / 100_000,
+                                "fp64_pipe": 0.370,
                                 "captured": "one launch on a 100,000-object sample of the workload"},
 }
 
@@ -131,8 +131,8 @@ WORKLOADS["thermal_wise_1m"] = ("thermal model, FRM with the four WISE bands and
                                 "lognormal median 0.14 sigma_ln 0.6, H U(8,20), G 0.15, "
                                 "emissivity 0.9), 2048-facet sphere")
 DEFAULT_N["thermal_wise_1m"] = 1_000_000
-# ncu sm__pipe_fp64_cycles_active of the FRM WISE kernel (one capture, 20k geometries)
-THERMAL_FP64_PIPE = 0.564
+# ncu sm__pipe_fp64_cycles_active of the FRM WISE kernel (one capture, 100k geometries)
+THERMAL_FP64_PIPE = 0.630
 WORKLOADS["stm_cov_1m"] = ("two-body state-transition matrices with covariance propagation, {n} "
                            "main-belt states, per-object spans U(-1000, 1000) d, one 6x6 "
                            "covariance per object (Phi C Phi^T)")
@@ -1544,8 +1544,8 @@ def run_thermal(args, world, rank, local):
         "roofline": {"bound": "fp64-transcendental", "achieved": None, "peak": None, "unit": None,
                      "frac": None, "traffic": None, "fp64_pipe_active_ncu": THERMAL_FP64_PIPE,
                      "note": "one exp per seen facet and band dominates and has no fixed flop "
-                             "count; the FP64 pipe is busy 56 % of the kernel's cycles with "
-                             "instruction issue the limit (ncu, 20k geometries)"},
+                             "count; the FP64 pipe is busy 63 % of the kernel's cycles with "
+                             "instruction issue the limit (ncu, 100k geometries)"},
         "neatm_same_inputs": {"ms_per_step": 1e3 * t_neatm / args.steps,
                               "value": world * n * args.steps / t_neatm, "unit": "geometries/s"},
         "cpu_baseline": {"value": k / cpu_s, "unit": "geometries/s", "cores": os.cpu_count(),
