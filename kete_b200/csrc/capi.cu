@@ -386,12 +386,13 @@ static void build_pool_plan(const FastPlan& P, PoolPlan& Q) {
         for (int64_t r = 1; r < S.n_rec; ++r)  // unscaled columns need one scale a series
             if (Q.km && g_pool_host[S.offset + r * S.rsize + 2] != Q.b[v].vscale) return;
     }
+    // the partner of an odd last body: where that body is (its centre with it, which says how the
+    // column is scaled), so that it changes no closest approach, without mass or extent
     PoolBody& D = Q.b[Q.n_body];
     D = Q.b[Q.n_body - 1];
     D.mass = D.j2m = 0.0;
     D.radius2 = -1.0;
     D.kind = FK_PLAIN;
-    D.chain = -1;
     // longest series first: the lanes of a warp then loop over similar counts
     std::stable_sort(Q.s, Q.s + Q.n_pos,
                      [](const PoolSeries& a, const PoolSeries& b) { return a.pairs > b.pairs; });

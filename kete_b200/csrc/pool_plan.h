@@ -18,8 +18,8 @@ struct PoolSeries {
 };
 // One body of the pooled force sum, in the fast plan's order (the bodies with velocities, then
 // the others; b[n_body] is a copy of the last one without mass or radius, the partner of an odd
-// one).  j2m: 1.5 J2 mass; vscale: the velocity series' scale; chain: cache slot of the centre whose position the body's is
-// relative to (-1: none).
+// one).  j2m: 1.5 J2 mass; vscale: the velocity series' scale; chain: cache slot of the centre
+// whose position the body's is relative to (-1: none).
 struct PoolBody {
     double mass, radius, radius2, j2m, vscale;
     int32_t slot, vslot, chain, naif_id, kind, pad_;
