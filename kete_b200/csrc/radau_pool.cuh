@@ -321,6 +321,7 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
                                                    const double v[3], PoolExact& ex,
                                                    double na = 0.0) {
     const int iv = sub & 1;
+    const double min_before = ex.min_r2;
     {
         const PoolBody& B = body[iv];
         double rp[3], rv[3];
@@ -356,10 +357,19 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
             term[(TERM_EARTH + 1) * NODE_G] = z2;
         }
     }
-    if (__any_sync(0xffffffffu, ex.impact_id != 0))
-#pragma unroll
-        for (int o = NODE_G; o < 32; o <<= 1)
-            ex.impact_id = max(ex.impact_id, __shfl_xor_sync(0xffffffffu, ex.impact_id, o));
+    // A struck body ends the list of those that count, for the impact (the first of the plan) as for
+    // the closest approach: the sub-lanes, each of which saw its own bodies, go through all of them
+    // again in the plan's order, as pool_forces does.
+    if (__any_sync(0xffffffffu, ex.impact_id != 0)) {
+        ex.impact_id = 0;
+        ex.min_r2 = min_before;
+#pragma unroll 1
+        for (int i = 0; i < n_body; ++i) {
+            double rp[3];
+            pool_body_position<KM>(body[i], x, col, stride, rp);
+            pool_checks(body[i], pool_r2(rp), exact, track, ex);
+        }
+    }
     if (track)
 #pragma unroll
         for (int o = NODE_G; o < 32; o <<= 1)
