@@ -36,6 +36,7 @@ extern "C" {
 #define KETE_B200_IMPACT 6
 #define KETE_B200_TIMEOUT 7
 #define KETE_B200_CHECKPOINT_FULL 8  /* checkpoint capacity too small; ckpt_count says how many */
+#define KETE_B200_CHECKPOINT_MISMATCH 9  /* adjoint: a replayed block does not lead to the next checkpoint */
 
 /* doubles per checkpoint of kete_b200_propagate_n_body_checkpointed */
 #define KETE_B200_CHECKPOINT_DOUBLES 36
@@ -387,10 +388,10 @@ int kete_b200_set_step_limit(int64_t max_steps);
 int kete_b200_set_sensitivity_form(int form);
 
 /* Form of the adjoint pass's replays (kete_b200_propagate_n_body_adjoint; no counterpart in the
- * reference): 0 (default) = every checkpoint block of every object re-run in one parallel
- * launch before the sweep, when their records fit a bounded library scratch (8 GiB; else as
- * 1); 1 = the sweep re-runs each block itself, just before transposing it.  Both give the same
- * gradients bit for bit (with the asteroid masses to rounding). */
+ * reference).  The checkpoint blocks are re-run from the last to the first in passes, as many of
+ * every object in one parallel launch as a bounded library scratch holds, and transposed by a
+ * sweep after each: 0 (default) = 8 GiB of scratch, most often one pass; 1 = 64 MiB (but a block
+ * of every object at least, 4,896 bytes each).  Both give the same gradients bit for bit. */
 int kete_b200_set_adjoint_form(int form);
 
 /* Form of the field checks (kete_b200_fov_check_visible and the schedule built on it; no

@@ -26,6 +26,7 @@ from .state import Frames
 
 
 CHECKPOINT_FULL = 8
+CHECKPOINT_MISMATCH = 9  # adjoint status: a replayed block does not lead to the next checkpoint
 SENS_CK_ATTEMPTS = 16
 
 
@@ -56,10 +57,9 @@ def set_sensitivity_form(form: int = 0):
 
 
 def set_adjoint_form(form: int = 0):
-    """Form of the adjoint pass's replays (kete_b200_set_adjoint_form): 0 = every checkpoint
-    block replayed in one parallel launch before the sweep (default, when the records fit the
-    library's bounded scratch); 1 = the sweep re-runs each block just before transposing it.
-    The gradients are identical."""
+    """Form of the adjoint pass's replays (kete_b200_set_adjoint_form): 0 = as many checkpoint
+    blocks at a time as 8 GiB of library scratch hold (default, most often all of them); 1 =
+    64 MiB, in more passes.  The gradients are identical."""
     L = _lib.lib()
     L.kete_b200_set_adjoint_form.argtypes = [ctypes.c_int]
     _lib.check(L.kete_b200_set_adjoint_form(int(form)))

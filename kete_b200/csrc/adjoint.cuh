@@ -11,9 +11,11 @@
 // b is scaled from (predict_b_row, radau.cuh).
 //
 // Backward (nbody_sens_backward_kernel): the segments and their checkpoint blocks are taken
-// in reverse.  A block is re-run from its checkpoint with the same step code, recording for
-// every attempt its start state, the step size used, its iteration count and the b of its
-// last corrector iteration.  The attempts are then transposed, last first.  For one attempt
+// in reverse.  A block is re-run from its checkpoint by the step code that ran it (the checkpoint
+// says which: these kernels or the pooled ones of sens_pool.cuh, whose sums may round otherwise;
+// another rounding changes which attempts are retried, and a block of so many attempts would
+// end elsewhere than the next begins), recording for every attempt its start state, the step
+// size used, its iteration count and the b of its last corrector iteration.  The attempts are then transposed, last first.  For one attempt
 // with M iterations (step size and iteration count held fixed):
 //   x' = x + h v + h^2 (a/2 + W.b^M),  v' = v + h (a + U.b^M),  a' = F(x', v')
 //   b^m = P (E^m - a),  E^m_j = F(X_j(b^(m-1)), V_j(b^(m-1))),  P = C_MAT . (divided differences)
@@ -44,7 +46,9 @@ enum SensPhase : int { SP_BEGIN = 0, SP_EXACT_INIT = 1, SP_ITER = 2, SP_EXACT_ST
 //   [3] record: 1 if the attempt converged  [4..6] x  [7..9] v  [10..12] a  [13..33] b
 //   [34] checkpoint: the previous step's h when b is to be predicted, else 0;
 //        record: the predictor's scale q used at the attempt's start, else 0
+//   [35] checkpoint: SENS_BY_POOL when the pooled kernels ran the object, else SENS_BY_NODES
 static_assert(SENS_STRIDE == 36, "checkpoint layout");
+constexpr double SENS_BY_NODES = 0.0, SENS_BY_POOL = 1.0;
 
 struct SensGroup {  // one object's integration state, identical in every lane of its group
     double t, tf, h, next_h, h_prev;
@@ -68,6 +72,7 @@ __device__ __forceinline__ void sens_store_state(double* dst, const SensGroup& G
         dst[1] = G.h;
         dst[2] = w2;
         dst[34] = G.predict ? G.h_prev : 0.0;
+        dst[35] = SENS_BY_NODES;
     } else if (lane == 1) {
         dst[4] = G.x[0]; dst[5] = G.x[1]; dst[6] = G.x[2];
     } else if (lane == 2) {
@@ -432,6 +437,7 @@ struct SensReplayPolicy {
     int na;       // attempts recorded
     int lane;
     double* sb;
+    bool ended = false;  // the replay reached the segment's end
 
     __device__ bool begin_attempt(SensGroup& G) {
         sens_store_state(rec + (size_t)na * SENS_STRIDE, G, sb, lane, 0.0);
@@ -461,9 +467,34 @@ struct SensReplayPolicy {
     }
     __device__ void segment_end(SensGroup& G) {
         sens_store_state(rec + (size_t)na * SENS_STRIDE, G, sb, lane, 0.0);
+        ended = true;
         G.phase = SP_PAUSE;
     }
 };
+
+// How many checkpoint blocks an object has.
+__device__ __forceinline__ int sens_block_count(const SensArgs& a, int64_t obj) {
+    return min(max(a.ckpt_count[obj], 0), a.ckpt_cap);
+}
+
+// The checkpoint that block cb of an object is followed by, null for the last of its segment k.
+__device__ __forceinline__ const double* sens_next_checkpoint(const SensArgs& a, int64_t obj, int k,
+                                                              int cb) {
+    const int end = k + 1 < a.n_epochs ? a.ckpt_seg[(int64_t)(k + 1) * a.n + obj]
+                                        : sens_block_count(a, obj);
+    return cb + 1 < end ? a.ckpt + ((size_t)obj * a.ckpt_cap + cb + 1) * SENS_STRIDE : nullptr;
+}
+
+// Whether a replayed block that stopped at t, x (ended: at its segment's end) leads to the next
+// checkpoint.  The replay of a block by the code that ran it is exact; a checkpoint of other
+// inputs, or one whose rounding changed a retry, is off by a good part of a step.
+__device__ __forceinline__ bool sens_block_follows(const double* next, bool ended, double t,
+                                                   const double* x) {
+    if (ended || !next) return ended && !next;
+    constexpr double TOL = 1e-6;  // days, AU
+    return fabs(t - next[0]) < TOL && fabs(x[0] - next[4]) < TOL && fabs(x[1] - next[5]) < TOL &&
+           fabs(x[2] - next[6]) < TOL;
+}
 
 // Jacobian of the force at one point: J (3 x 6) = d a / d(x, v) and jp (3 x 2) = d a / d(A1, A2),
 // in closed form inside the fast plan's window, by dual numbers outside it.  Out of line: one
@@ -496,10 +527,10 @@ static __device__ __noinline__ int sens_jacobian(TangentForce& T, double t, cons
     return ST_OK;
 }
 
-// Re-run checkpoint block `c` (its segment ends at tf) with the step code, recording every
-// attempt into rec (SENS_CK_ATTEMPTS + 1 records).  Returns ST_OK with the attempt count in na,
-// or the failure.
-__device__ __forceinline__ int sens_replay_block(const double* c, double tf, double* rec,
+// Re-run checkpoint block `c` (its segment ends at tf; next: the checkpoint it leads to, null for
+// the last block) with the step code, recording every attempt into rec (SENS_CK_ATTEMPTS + 1
+// records).  Returns ST_OK with the attempt count in na, or the failure.
+__device__ __forceinline__ int sens_replay_block(const double* c, double tf, const double* next, double* rec,
                                                  SpkForce& F, const double* nrow, double* sb,
                                                  double* se, int lane, int comp, unsigned gmask,
                                                  int warp_lane, int max_rounds, EphCache& C,
@@ -533,16 +564,17 @@ __device__ __forceinline__ int sens_replay_block(const double* c, double tf, dou
     na = P.na;
     __syncwarp(gmask);  // the records are complete and visible to the group
     if (G.phase != SP_PAUSE) return G.rc != ST_OK ? G.rc : ST_TIMEOUT;
-    return ST_OK;
+    return sens_block_follows(next, P.ended, G.t, G.x) ? ST_OK : ST_CHECKPOINT_MISMATCH;
 }
 
-// The replays of every checkpoint block of every object at once, before the adjoint sweep:
+// The replays of a pass's checkpoint blocks of every object at once, before the sweep over them:
 // a block's replay depends only on its checkpoint, so groups of 8 lanes re-run the blocks in
 // parallel and store each block's attempt records (a.rec_all) and outcome (a.rep_count: the
 // attempt count, or -1 - status on failure) for the sweep to read.  The grid is persistent:
 // each group takes the next block from a queue (a.rep_first[n + 2]) in the dense order of
 // a.rep_first (sens_replay_offsets_kernel), so groups that finish early take more blocks
-// instead of leaving their thread block's other groups to run alone.
+// instead of leaving their thread block's other groups to run alone.  After the pooled replay
+// (a.pending) it takes the blocks left to it, and ends at once when there are none.
 template <int MINB>
 __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(SensArgs a) {
     __shared__ double s_node[8 * NODE_ROW_S];
@@ -556,6 +588,7 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(Sen
     const int64_t n = a.n;
     const int64_t total = a.rep_first[n];
     int32_t* queue = a.rep_first + n + 2;
+    if (a.pending && a.rep_first[n + 3] == 0) return;
     double* sb = s_b[threadIdx.x / SG];
     double* se = s_e[threadIdx.x / SG];
     const int comp = lane % 3;
@@ -575,8 +608,9 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(Sen
             else hi = mid;
         }
         const int64_t obj = lo;
-        const int cb = (int)(idx - a.rep_first[obj]);
-        const int64_t item = obj * a.ckpt_cap + cb;  // the sweep's layout of records and counts
+        const int at = (int)(idx - a.rep_first[obj]);
+        const int cb = sens_pass_first(sens_block_count(a, obj), a.pass, a.window) + at;
+        const int64_t item = obj * a.window + at;  // the sweep's layout of records and counts
         if (a.pending && a.rep_count[item] != SENS_PENDING) continue;
         int k = 0;  // the epoch segment holding block cb
         while (k + 1 < a.n_epochs && a.ckpt_seg[(int64_t)(k + 1) * n + obj] <= cb) ++k;
@@ -594,22 +628,21 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(Sen
         double* rec = a.rec_all + (size_t)item * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE;
         const double* c = a.ckpt + ((size_t)obj * a.ckpt_cap + cb) * SENS_STRIDE;
         int na = 0;
-        const int rc = sens_replay_block(c, a.epochs[k], rec, F, nrow, sb, se, lane, comp, gmask,
+        const int rc = sens_replay_block(c, a.epochs[k], sens_next_checkpoint(a, obj, k, cb), rec, F, nrow, sb, se, lane, comp, gmask,
                                          warp_lane, a.max_loops * 12, C, na);
         if (lane == 0) a.rep_count[item] = rc == ST_OK ? na : -1 - rc;
         __syncwarp(gmask);  // sb, se and the cache are reused by the group's next block
     }
 }
 
-// REPLAY: the sweep re-runs each block itself (the records did not fit the up-front replay's
-// scratch); otherwise it reads the records nbody_sens_replay_kernel wrote, and carries no
-// step code (a smaller kernel with fewer registers).
-template <int MINB, bool REPLAY>
+// The sweep over a pass's blocks, from the records of the replays before it; it carries no step
+// code (a smaller kernel with fewer registers).  PASSES: more passes than one; the state goes
+// through a.sweep from one to the next: the adjoint of the state and of b, the lanes' sums for
+// A1 and A2, and the segment it is in (-1: done).  The values are those of a single pass.
+template <int MINB, bool PASSES>
 __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_backward_kernel(SensArgs a) {
     __shared__ double s_node[8 * NODE_ROW_S];
     __shared__ double s_P[49];
-    __shared__ double s_b[SENS_BLOCK / SG][21];
-    __shared__ double s_e[SENS_BLOCK / SG][SG * 3];
     __shared__ double s_lb[SENS_BLOCK / SG][21];
     __shared__ double s_t[SENS_BLOCK / SG][7 * 6];
     sens_load_nodes(s_node);
@@ -626,30 +659,20 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_backward_kernel(S
         if (lane < 8) a.out_grad[(int64_t)lane * n + obj] = nan;
         return;
     }
-    double* sb = s_b[threadIdx.x / SG];
-    double* se = s_e[threadIdx.x / SG];
     double* slb = s_lb[threadIdx.x / SG];
     double* stx = s_t[threadIdx.x / SG];
-    const int comp = lane % 3;
     const double* nrow = s_node + (lane < 7 ? lane + 1 : 7) * NODE_ROW_S;
-    double* rec_own = a.rec + (size_t)obj * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE;
     const double* ck = a.ckpt + (size_t)obj * a.ckpt_cap * SENS_STRIDE;
 
-    SpkForce F;
-    F.n_force = a.n_force;
-    F.ng.base = a.nongrav ? a.nongrav + obj : nullptr;
-    F.ng.stride = n;
-    F.ng.kind = a.nongrav ? (int)a.nongrav[obj] : 0;
-    F.impact_id = 0;
-    F.min_dist = 1e300;
-    F.min_id = 0;
     TangentForce T;
     T.n_force = a.n_force;
-    T.ng = F.ng;
+    T.ng.base = a.nongrav ? a.nongrav + obj : nullptr;
+    T.ng.stride = n;
+    T.ng.kind = a.nongrav ? (int)a.nongrav[obj] : 0;
     T.impact_id = 0;
     T.min_dist = 1e300;
     // per-lane body positions in dynamic shared memory (EPH_CACHE x SENS_BLOCK doubles,
-    // launch_sens_backward), shared by the replay and the Jacobian rounds
+    // launch_sens_backward)
     extern __shared__ double s_dyn[];
     const FastPlan& plan = a.n_force == c_eph.n_force_planets ? c_eph.fast_planets : c_eph.fast_all;
     EphCache C{s_dyn + threadIdx.x, SENS_BLOCK,
@@ -661,54 +684,82 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_backward_kernel(S
     double lx[3] = {0, 0, 0}, lv[3] = {0, 0, 0}, la[3];
     double dA0 = 0.0, dA1 = 0.0;
     int fail = ST_OK;
-    const int n_ck = a.ckpt_count[obj];
-    const int max_rounds = a.max_loops * 12;
-
-    for (int k = a.n_epochs - 1; k >= 0 && fail == ST_OK; --k) {
-        // seed: dL/d(state at epoch k), caller frame -> integration frame (x_eq = R x)
-        const double* sd = a.seed + (int64_t)k * 6 * n;
+    const int n_ck = sens_block_count(a, obj);
+    // the pass's blocks: from block first up to the one before the last pass's
+    const int first = PASSES ? sens_pass_first(n_ck, a.pass, a.window) : 0;
+    const int above = PASSES && a.pass > 0 ? sens_pass_first(n_ck, a.pass - 1, a.window) : n_ck;
+    double* saved = PASSES ? a.sweep + (size_t)obj * SENS_SWEEP_STATE : nullptr;
+    int k = a.n_epochs - 1;
+    bool resumed = false;  // in the middle of segment k
+    if (PASSES && a.pass > 0) {
+        k = (int)saved[46];
+        resumed = true;
+        if (k < 0) return;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            double sx = 0.0, sv = 0.0;
+            lx[c] = saved[c];
+            lv[c] = saved[3 + c];
+            la[c] = saved[6 + c];
+        }
+        dA0 = saved[9 + lane];
+        dA1 = saved[17 + lane];
+        if (lane < 7)
 #pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                sx += R[c][q] * sd[q * n + obj];
-                sv += R[c][q] * sd[(3 + q) * n + obj];
-            }
-            lx[c] += sx;
-            lv[c] += sv;
-            la[c] = 0.0;  // the acceleration at the segment end feeds nothing
-        }
-        if (lane < 7) {  // b restarts at zero in the next segment: no adjoint flows back
-            slb[lane] = 0.0;
-            slb[7 + lane] = 0.0;
-            slb[14 + lane] = 0.0;
-        }
+            for (int c = 0; c < 3; ++c) slb[7 * c + lane] = saved[25 + 7 * c + lane];
         __syncwarp(gmask);
+    }
+
+    for (; k >= 0 && fail == ST_OK; --k) {
+        if (!resumed) {
+            // seed: dL/d(state at epoch k), caller frame -> integration frame (x_eq = R x)
+            const double* sd = a.seed + (int64_t)k * 6 * n;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                double sx = 0.0, sv = 0.0;
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    sx += R[c][q] * sd[q * n + obj];
+                    sv += R[c][q] * sd[(3 + q) * n + obj];
+                }
+                lx[c] += sx;
+                lv[c] += sv;
+                la[c] = 0.0;  // the acceleration at the segment end feeds nothing
+            }
+            if (lane < 7) {  // b restarts at zero in the next segment: no adjoint flows back
+                slb[lane] = 0.0;
+                slb[7 + lane] = 0.0;
+                slb[14 + lane] = 0.0;
+            }
+            __syncwarp(gmask);
+        }
+        resumed = false;
         const int c0 = a.ckpt_seg[(int64_t)k * n + obj];
         const int c1 = k + 1 < a.n_epochs ? a.ckpt_seg[(int64_t)(k + 1) * n + obj] : n_ck;
-        const double tf = a.epochs[k];
-        for (int cb = c1 - 1; cb >= c0 && fail == ST_OK; --cb) {
-            // ---- the block's attempt records: replayed up front, or re-run here ----
-            const double* c = ck + (size_t)cb * SENS_STRIDE;
-            int na = 0;
-            double* rec = rec_own;
-            if (!REPLAY) {
-                const size_t item = (size_t)obj * a.ckpt_cap + cb;
-                rec = a.rec_all + item * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE;
-                const int cnt = a.rep_count[item];
-                if (cnt < 0) {
-                    fail = -1 - cnt;
-                    break;
+        for (int cb = min(above, c1) - 1; cb >= c0 && fail == ST_OK; --cb) {
+            if (PASSES && cb < first) {  // the next pass goes on here
+                if (lane == 0) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        saved[c] = lx[c];
+                        saved[3 + c] = lv[c];
+                        saved[6 + c] = la[c];
+                    }
+                    saved[46] = (double)k;
                 }
-                na = cnt;
-            } else {
-                const int rrc = sens_replay_block(c, tf, rec, F, nrow, sb, se, lane, comp, gmask,
-                                                  warp_lane, max_rounds, C, na);
-                if (rrc != ST_OK) {
-                    fail = rrc;
-                    break;
-                }
+                saved[9 + lane] = dA0;
+                saved[17 + lane] = dA1;
+                if (lane < 7)
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) saved[25 + 7 * c + lane] = slb[7 * c + lane];
+                return;
+            }
+            // ---- the block's attempt records ----
+            const size_t item = (size_t)obj * a.window + (cb - first);
+            const double* rec = a.rec_all + item * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE;
+            const int na = a.rep_count[item];
+            if (na < 0) {
+                fail = -1 - na;
+                break;
             }
             // ---- transpose the attempts, last first ----
             for (int s = na - 1; s >= 0; --s) {
@@ -900,6 +951,7 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_backward_kernel(S
         g[6 * n + obj] = fail == ST_OK ? dA0 : nan;
         g[7 * n + obj] = fail == ST_OK ? dA1 : nan;
         if (a.grad_status) a.grad_status[obj] = fail;
+        if (PASSES) saved[46] = -1.0;
     }
 }
 

@@ -1486,28 +1486,22 @@ int kete_b200_propagate_n_body_adjoint(int64_t n, int n_epochs, const double* ep
     a.max_loops = g_launch.max_loops;
     a.pool_slots = pool_slots(a.n_force);
     if (S.rc) return S.rc;
-    // per-object attempt records of the block being transposed (library scratch)
-    void* rec;
-    if ((rc = staging(*ds, 33, (size_t)n * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE * sizeof(double), &rec)))
+    // the attempt records of as many blocks of every object as a bounded library scratch holds,
+    // and what the sweep carries between passes when that is not all of them
+    const size_t block_bytes = (size_t)n * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE * sizeof(double);
+    const size_t bound = g_launch.adjoint_form == 1 ? ADJOINT_SMALL_BYTES : ADJOINT_REPLAY_BYTES;
+    a.window = (int)std::min<size_t>(ckpt_capacity, std::max<size_t>(1, bound / block_bytes));
+    void *ra, *rn, *rf, *sw = nullptr;
+    if ((rc = staging(*ds, 35, block_bytes * a.window, &ra)) ||
+        (rc = staging(*ds, 36, (size_t)n * a.window * sizeof(int32_t), &rn)) ||
+        (rc = staging(*ds, 34, ((size_t)n + 4) * sizeof(int32_t), &rf)) ||
+        (a.window < ckpt_capacity &&
+         (rc = staging(*ds, 33, (size_t)n * SENS_SWEEP_STATE * sizeof(double), &sw))))
         return rc;
-    a.rec = (double*)rec;
-    // the records of every checkpoint block, replayed in parallel before the sweep, when they
-    // fit a bounded scratch (else each block is re-run inside the sweep)
-    const size_t all_bytes =
-        (size_t)n * ckpt_capacity * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE * sizeof(double);
-    a.rec_all = nullptr;
-    a.rep_count = nullptr;
-    a.rep_first = nullptr;
-    if (g_launch.adjoint_parallel_replay && all_bytes <= ADJOINT_REPLAY_BYTES) {
-        void *ra, *rn, *rf;
-        if ((rc = staging(*ds, 35, all_bytes, &ra)) ||
-            (rc = staging(*ds, 36, (size_t)n * ckpt_capacity * sizeof(int32_t), &rn)) ||
-            (rc = staging(*ds, 34, ((size_t)n + 3) * sizeof(int32_t), &rf)))
-            return rc;
-        a.rec_all = (double*)ra;
-        a.rep_count = (int32_t*)rn;
-        a.rep_first = (int32_t*)rf;
-    }
+    a.rec_all = (double*)ra;
+    a.rep_count = (int32_t*)rn;
+    a.rep_first = (int32_t*)rf;
+    a.sweep = (double*)sw;
     if ((rc = launch_sens_backward(a, st))) return rc;
     return S.finish();
 }
@@ -1766,7 +1760,7 @@ int kete_b200_set_sensitivity_form(int form) {
 int kete_b200_set_adjoint_form(int form) {
     if (form != 0 && form != 1) return set_error(KETE_B200_E_ARGUMENT, "adjoint form is 0 or 1");
     std::lock_guard<std::mutex> lk(g_mu);
-    g_launch.adjoint_parallel_replay = form == 0;
+    g_launch.adjoint_form = form;
     return 0;
 }
 

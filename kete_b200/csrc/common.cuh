@@ -19,6 +19,7 @@ enum Status : int32_t {
     ST_TIMEOUT = 7,  // a bounded device loop ran out of iterations
     ST_PENDING = -1,  // internal: left by one kernel of a call to the next
     ST_CHECKPOINT_FULL = 8,  // more checkpoints were needed than the caller provided
+    ST_CHECKPOINT_MISMATCH = 9,  // a replayed checkpoint block does not lead to the next one
 };
 
 enum Frame : int32_t { FRAME_EQUATORIAL = 1, FRAME_ECLIPTIC = 2 };

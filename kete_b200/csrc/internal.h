@@ -134,10 +134,10 @@ struct LaunchConfig {
     int max_loops_long = 1 << 24;  // system integration (every batch's whole span)
     int sens_form = 0;  // forward sensitivities: 0 node-parallel, 1 one object per thread
     int fov_form = 0;   // field checks: 0 linear screen + two-body pass, 1 one fused pass
-    int adjoint_parallel_replay = 1;  // adjoint: replay every checkpoint block up front
+    int adjoint_form = 0;  // scratch of the adjoint's replays: 0 ADJOINT_REPLAY_BYTES, 1 ADJOINT_SMALL_BYTES
 };
-// scratch bound of the adjoint's up-front replay (every block's attempt records)
-constexpr size_t ADJOINT_REPLAY_BYTES = size_t(8) << 30;
+// bounds of the attempt records that the adjoint holds at a time (a block of every object at least)
+constexpr size_t ADJOINT_REPLAY_BYTES = size_t(8) << 30, ADJOINT_SMALL_BYTES = size_t(64) << 20;
 LaunchConfig& launch_config();
 // What the allocation-free entry point launches: the node variant in cfg.nodes_variant, the
 // variant with the general ephemeris evaluation, and the window of launch_span_order.
@@ -201,18 +201,28 @@ struct SensArgs {
     const double* seed;  // n_epochs x 6 x n: dL/d(state at each epoch) (adjoint)
     double* out_grad;    // 8 x n: dL/d(pos0, vel0, A1, A2) (adjoint)
     int32_t* grad_status;  // n or null (adjoint)
-    double* rec;         // n x (SENS_CK_ATTEMPTS + 1) x SENS_STRIDE scratch (adjoint)
-    double* rec_all;     // n x ckpt_cap x (SENS_CK_ATTEMPTS + 1) x SENS_STRIDE, or null: the
-                         // records of every block, replayed up front (adjoint)
-    int32_t* rep_count;  // n x ckpt_cap: attempts of each replayed block, -1 - status on failure
-    int32_t* rep_first;  // n + 3 (with rec_all): exclusive prefix sums of the blocks to replay
-                         // per object (the replay takes the blocks in this dense order), then
-                         // the queue counters of the pooled and the general replay
+    // adjoint scratch.  The sweep goes backwards in passes of `window` blocks an object: pass p
+    // replays blocks sens_pass_first(count, p) on, of which there are at most `window`, and
+    // transposes them; one pass when window >= ckpt_cap.
+    int window, pass;
+    double* rec_all;     // n x window x (SENS_CK_ATTEMPTS + 1) x SENS_STRIDE: the pass's records
+    int32_t* rep_count;  // n x window: attempts of each replayed block, -1 - status on failure
+    int32_t* rep_first;  // n + 4: exclusive prefix sums of the pass's blocks per object (the replays
+                         // take the blocks in this dense order), then the queue counters of the
+                         // pooled and the general replay and how many blocks the first left
+    double* sweep;       // n x SENS_SWEEP_STATE: the sweep's state between passes
     int max_loops;
     int pool_slots;  // doubles of a pooled cache column, 0: the pooled form cannot serve
     int pending;     // only the objects whose status is ST_PENDING, the blocks marked SENS_PENDING
 };
 constexpr int SENS_PENDING = -2147483647 - 1;  // rep_count of a block left to the general replay
+constexpr int SENS_SWEEP_STATE = 48;
+// The first block that pass `pass` of an object with `count` blocks takes (the passes go from the
+// last block to the first).
+inline __host__ __device__ int sens_pass_first(int count, int pass, int window) {
+    const int64_t first = count - (pass + (int64_t)1) * window;
+    return first > 0 ? (int)first : 0;
+}
 // sens_pool.cu: the passes on the warp-pooled step machinery, for what lies inside the window
 int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream);
 int launch_sens_pool_replay(const SensArgs& a, cudaStream_t stream);

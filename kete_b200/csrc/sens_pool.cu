@@ -58,13 +58,13 @@ int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream) {
     return launched(1, "sens_pool_forward_kernel launch");
 }
 
-// Persistent grids; a.n * a.ckpt_cap bounds the blocks to replay (about twice what there are).
+// Persistent grids; a.n * a.window bounds the blocks to replay.
 int launch_sens_pool_replay(const SensArgs& a, cudaStream_t stream) {
     int dev = 0, sms = 0, per_sm = 0;
     int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc || (rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")))
         return rc;
-    const int64_t most = a.n * (int64_t)a.ckpt_cap;
+    const int64_t most = a.n * (int64_t)a.window;
     const bool wide = most <= 8192;
     const auto k4 = sens_pool_replay_kernel<4, WIDE_BLOCK, 12>;
     const auto k1 = sens_pool_replay_kernel<1, SENS_POOL_BLOCK, 3>;

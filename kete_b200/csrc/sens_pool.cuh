@@ -10,8 +10,9 @@
 // in shared memory.  S = 4 gives an object a warp (few objects: every step is waited for), S = 1
 // eight lanes (many checkpoint blocks).
 //
-// The kernels take what lies inside the fast plan's window; the others are marked ST_PENDING (a
-// replayed block: SENS_PENDING) and left to the kernels of adjoint.cuh and stm_nodes.cuh.
+// The forward kernels take the objects inside the fast plan's window and mark the others ST_PENDING
+// for the kernels of adjoint.cuh and stm_nodes.cuh; the replays take the blocks whose checkpoint
+// says that the forward pass was the one here, and mark the others SENS_PENDING.
 #pragma once
 #include "adjoint.cuh"
 #include "radau_pool.cuh"
@@ -414,6 +415,7 @@ __device__ __forceinline__ void sens_pool_store_state(const SensPoolGroup& G, do
         dst[1] = st[ST_H];
         dst[2] = w2;
         dst[34] = predict ? st[ST_HP] : 0.0;
+        dst[35] = SENS_BY_POOL;
     } else if (lane < 4) {
         const int from = lane == 1 ? ST_X : (lane == 2 ? ST_V : ST_A);
 #pragma unroll
@@ -511,7 +513,9 @@ struct SensPoolReplay {
     int64_t total;
     int64_t item = 0;
     double* rec = nullptr;
+    const double* after = nullptr;  // the checkpoint that the block leads to
     int na = 0;
+    bool ended = false;
 
     __device__ bool next(SensPoolGroup& G, bool& resume, int& failures, bool& predict) {
         const int64_t n = a.n;
@@ -528,21 +532,28 @@ struct SensPoolReplay {
                 else hi = mid;
             }
             const int64_t obj = lo;
-            const int cb = (int)(idx - a.rep_first[obj]);
-            item = obj * a.ckpt_cap + cb;
+            const int at = (int)(idx - a.rep_first[obj]);
+            const int cb = sens_pass_first(sens_block_count(a, obj), a.pass, a.window) + at;
+            item = obj * a.window + at;
             int e0 = 0, e1 = a.n_epochs;  // the epoch segment: the last one starting at or before cb
             while (e1 - e0 > 1) {
                 const int mid = (e0 + e1) >> 1;
                 if (a.ckpt_seg[(int64_t)mid * n + obj] <= cb) e0 = mid;
                 else e1 = mid;
             }
-            const double* c = a.ckpt + (size_t)item * SENS_STRIDE;
+            const double* c = a.ckpt + ((size_t)obj * a.ckpt_cap + cb) * SENS_STRIDE;
             const double t = c[0], tf = a.epochs[e0];
+            // (the window: checkpoints of another ephemeris than the present one)
             const FastPlan& plan = a.n_force == c_eph.n_force_planets ? c_eph.fast_planets : c_eph.fast_all;
-            if (!in_window(t, tf, plan.lo, plan.hi)) {
-                if (G.leader) a.rep_count[item] = SENS_PENDING;
+            if (c[35] != SENS_BY_POOL || !in_window(t, tf, plan.lo, plan.hi)) {
+                if (G.leader) {
+                    a.rep_count[item] = SENS_PENDING;
+                    atomicAdd(a.rep_first + n + 3, 1);
+                }
                 continue;
             }
+            after = sens_next_checkpoint(a, obj, e0, cb);
+            ended = false;
             G.ng.base = a.nongrav ? a.nongrav + obj : nullptr;
             G.ng.stride = n;
             G.ng.kind = a.nongrav ? (int)a.nongrav[obj] : 0;
@@ -572,7 +583,11 @@ struct SensPoolReplay {
         }
     }
     __device__ void job_done(SensPoolGroup& G) {
-        if (G.leader) a.rep_count[item] = G.rc == ST_OK ? na : -1 - G.rc;
+        if (!G.leader) return;
+        int rc = G.rc;
+        if (rc == ST_OK && !sens_block_follows(after, ended, G.st[ST_T], G.st + ST_X))
+            rc = ST_CHECKPOINT_MISMATCH;
+        a.rep_count[item] = rc == ST_OK ? na : -1 - rc;
     }
     __device__ bool begin_attempt(SensPoolGroup& G, int, int, bool predict) {
         sens_pool_store_state(G, rec + (size_t)na * SENS_STRIDE, 0.0, predict);
@@ -602,6 +617,7 @@ struct SensPoolReplay {
     }
     __device__ bool segment_end(SensPoolGroup& G, int&, bool& predict) {
         sens_pool_store_state(G, rec + (size_t)na * SENS_STRIDE, 0.0, predict);
+        ended = true;
         return false;
     }
 };
