@@ -821,17 +821,16 @@ static bool launch_is_default() {
     return g_launch.nodes_variant == d.nodes_variant && g_launch.nodes_refill == d.nodes_refill;
 }
 
-// Doubles of a pooled cache column, 0 where the plan cannot serve.
-static int pool_slots(int n_force) {
-    const PoolPlan& Q = n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
-    return Q.ok ? Q.n_slot : 0;
-}
-
-// What the pooled kernels read besides the plan in constant memory.
-static void set_pool(NBodyArgs& a, double lo, double hi) {
+// What the pooled kernels read besides the plan in constant memory (no columns where the plan
+// cannot serve).
+template <class A>
+static void set_pool(A& a) {
     const PoolPlan& Q = a.n_force == g_eph.n_force_planets ? g_plans.planets : g_plans.all;
-    a.pool_slots = Q.n_slot;
+    a.pool_slots = Q.ok ? Q.n_slot : 0;
     a.pool_km = Q.km;
+}
+static void set_pool(NBodyArgs& a, double lo, double hi) {
+    set_pool(a);
     a.lo = lo;
     a.hi = hi;
 }
@@ -1387,7 +1386,7 @@ int kete_b200_propagate_n_body_stm(int64_t n, const double* pos, const double* v
     a.out_stm = S.out(out_stm, (size_t)n_epochs * 48 * n);
     a.status = S.out(status, (size_t)n);
     a.max_loops = g_launch.max_loops;
-    a.pool_slots = pool_slots(a.n_force);
+    set_pool(a);
     if (S.rc) return S.rc;
     if ((rc = launch_nbody_stm(a, g_launch.sens_form, st))) return rc;
     return S.finish();
@@ -1439,7 +1438,7 @@ int kete_b200_propagate_n_body_checkpointed(int64_t n, const double* pos, const 
     a.ckpt_count = S.out(ckpt_count, (size_t)n);
     a.ckpt_seg = S.out(ckpt_segment, (size_t)n_epochs * n);
     a.max_loops = g_launch.max_loops;
-    a.pool_slots = pool_slots(a.n_force);
+    set_pool(a);
     if (S.rc) return S.rc;
     if ((rc = launch_sens_forward(a, st))) return rc;
     return S.finish();
@@ -1484,7 +1483,7 @@ int kete_b200_propagate_n_body_adjoint(int64_t n, int n_epochs, const double* ep
     a.out_grad = S.out(out_grad, 8 * (size_t)n);
     a.grad_status = S.out(grad_status, (size_t)n);
     a.max_loops = g_launch.max_loops;
-    a.pool_slots = pool_slots(a.n_force);
+    set_pool(a);
     if (S.rc) return S.rc;
     // the attempt records of as many blocks of every object as a bounded library scratch holds,
     // and what the sweep carries between passes when that is not all of them

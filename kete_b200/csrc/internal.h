@@ -172,6 +172,7 @@ struct StmArgs {
     int32_t* status;
     int max_loops;
     int pool_slots;  // doubles of a pooled cache column, 0: the pooled form cannot serve
+    int pool_km;     // unscaled columns (PoolPlan::km)
     int pending;     // only the objects whose status is ST_PENDING
 };
 // form: 0 = node-parallel (8 lanes per object), 1 = one object per thread
@@ -213,6 +214,7 @@ struct SensArgs {
     double* sweep;       // n x SENS_SWEEP_STATE: the sweep's state between passes
     int max_loops;
     int pool_slots;  // doubles of a pooled cache column, 0: the pooled form cannot serve
+    int pool_km;     // unscaled columns (PoolPlan::km)
     int pending;     // only the objects whose status is ST_PENDING, the blocks marked SENS_PENDING
 };
 constexpr int SENS_PENDING = -2147483647 - 1;  // rep_count of a block left to the general replay

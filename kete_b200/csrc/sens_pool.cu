@@ -18,7 +18,7 @@ int upload_pool_plans_sens(const PoolPlans& p) {
 // Dynamic shared memory past 48 KB has to be allowed once per device (a function attribute, not
 // a stream operation).
 static int allow_smem(const void* kernel, int slot, int bytes) {
-    static std::atomic<unsigned long long> done[2];
+    static std::atomic<unsigned long long> done[4];
     int dev = 0;
     int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc) return rc;
@@ -42,14 +42,15 @@ using SharedStm = SensPoolShared<4, WIDE_BLOCK, STM_ROW>;
 // and 4.45; 730 days, 4096 objects: 14.06 and 8.96 (thread groups that replay per node: 12.8).
 constexpr int64_t SENS_WIDE_MAX = 1776;
 
-int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream) {
+template <bool KM>
+static int launch_forward(const SensArgs& a, cudaStream_t stream) {
     if (a.n <= SENS_WIDE_MAX) {
         const int smem = Shared4::doubles(a.pool_slots) * (int)sizeof(double);
-        sens_pool_forward_kernel<4, WIDE_BLOCK, 12><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
+        sens_pool_forward_kernel<4, WIDE_BLOCK, 12, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
     } else {
-        const auto kernel = sens_pool_forward_kernel<1, SENS_POOL_BLOCK, 3>;
+        const auto kernel = sens_pool_forward_kernel<1, SENS_POOL_BLOCK, 3, KM>;
         const int smem = Shared1::doubles(a.pool_slots) * (int)sizeof(double);
-        const int rc = allow_smem((const void*)kernel, 0,
+        const int rc = allow_smem((const void*)kernel, 2 * KM,
                                   Shared1::doubles(POOL_MAX_SLOTS) * (int)sizeof(double));
         if (rc) return rc;
         const int64_t grid = (a.n * NODE_G + SENS_POOL_BLOCK - 1) / SENS_POOL_BLOCK;
@@ -58,19 +59,24 @@ int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream) {
     return launched(1, "sens_pool_forward_kernel launch");
 }
 
+int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream) {
+    return a.pool_km ? launch_forward<true>(a, stream) : launch_forward<false>(a, stream);
+}
+
 // Persistent grids; a.n * a.window bounds the blocks to replay.
-int launch_sens_pool_replay(const SensArgs& a, cudaStream_t stream) {
+template <bool KM>
+static int launch_replay(const SensArgs& a, cudaStream_t stream) {
     int dev = 0, sms = 0, per_sm = 0;
     int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
     if (rc || (rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")))
         return rc;
     const int64_t most = a.n * (int64_t)a.window;
     const bool wide = most <= 8192;
-    const auto k4 = sens_pool_replay_kernel<4, WIDE_BLOCK, 12>;
-    const auto k1 = sens_pool_replay_kernel<1, SENS_POOL_BLOCK, 3>;
+    const auto k4 = sens_pool_replay_kernel<4, WIDE_BLOCK, 12, KM>;
+    const auto k1 = sens_pool_replay_kernel<1, SENS_POOL_BLOCK, 3, KM>;
     const int smem = (wide ? Shared4::doubles(a.pool_slots) : Shared1::doubles(a.pool_slots)) *
                      (int)sizeof(double);
-    if (!wide && (rc = allow_smem((const void*)k1, 1,
+    if (!wide && (rc = allow_smem((const void*)k1, 1 + 2 * KM,
                                   Shared1::doubles(POOL_MAX_SLOTS) * (int)sizeof(double))))
         return rc;
     const int block = wide ? WIDE_BLOCK : SENS_POOL_BLOCK;
@@ -86,14 +92,23 @@ int launch_sens_pool_replay(const SensArgs& a, cudaStream_t stream) {
     return launched(1, "sens_pool_replay_kernel launch");
 }
 
-int launch_sens_pool_stm(const StmArgs& a, cudaStream_t stream) {
+int launch_sens_pool_replay(const SensArgs& a, cudaStream_t stream) {
+    return a.pool_km ? launch_replay<true>(a, stream) : launch_replay<false>(a, stream);
+}
+
+template <bool KM>
+static int launch_stm(const StmArgs& a, cudaStream_t stream) {
     const int smem = SharedStm::doubles(a.pool_slots) * (int)sizeof(double);
     // Eight blocks an SM leave a thread 255 registers, which pays while that is one wave: 1021
     // objects 6.46 ms and 6.81 with twelve, 4096 objects 38.8 ms and 34.3
     // (sixteen: 38.4).
-    if (a.n <= 8 * 148) sens_pool_stm_kernel<8><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
-    else sens_pool_stm_kernel<12><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
+    if (a.n <= 8 * 148) sens_pool_stm_kernel<8, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
+    else sens_pool_stm_kernel<12, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
     return launched(1, "sens_pool_stm_kernel launch");
+}
+
+int launch_sens_pool_stm(const StmArgs& a, cudaStream_t stream) {
+    return a.pool_km ? launch_stm<true>(a, stream) : launch_stm<false>(a, stream);
 }
 
 }  // namespace kb

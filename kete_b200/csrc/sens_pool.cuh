@@ -8,7 +8,8 @@
 // whole warp for the seven node times and the step end (the exact evaluation reads the step end's
 // column, where every lane evaluated the same eleven records again), and a group's state lives
 // in shared memory.  S = 4 gives an object a warp (few objects: every step is waited for), S = 1
-// eight lanes (many checkpoint blocks).
+// eight lanes (many checkpoint blocks).  KM: unscaled columns for the plan with the asteroid masses,
+// as in radau_pool.cuh, so that the sums are the general kernels'.
 //
 // The forward kernels take the objects inside the fast plan's window and mark the others ST_PENDING
 // for the kernels of adjoint.cuh and stm_nodes.cuh; the replays take the blocks whose checkpoint
@@ -58,6 +59,7 @@ struct SensPoolGroup {
 
 // d force / d(x, v) and d force / d(A1, A2) from a cache column (TangentForce::jacobian_cached on
 // the pooled plan).
+template <bool KM>
 __device__ __forceinline__ void pool_jacobian(const PoolTables& T, const double* col, int stride,
                                               const NonGrav& ng, const double x[3],
                                               const double v[3], double J[18], double jp[6]) {
@@ -70,7 +72,7 @@ __device__ __forceinline__ void pool_jacobian(const PoolTables& T, const double*
     for (int i = 0; i < T.n_body; ++i) {
         const PoolBody& B = T.plan->b[i];
         double rp[3];
-        pool_relative(x, col + B.slot * stride, stride, rp);
+        pool_body_position<KM>(B, x, col, stride, rp);
         const double ir = rsqrt(pool_r2(rp));
         const double ir2 = ir * ir, kk = B.mass * ir2 * ir, k3 = 3.0 * kk * ir2;
         xx += k3 * rp[0] * rp[0] - kk;
@@ -85,7 +87,7 @@ __device__ __forceinline__ void pool_jacobian(const PoolTables& T, const double*
         TangentForce::j2_gradient(rp, ir, ir2, B.j2m * B.radius2, n, J);
         if (!vel) continue;
         double rv[3];
-        pool_relative(v, col + B.vslot * stride, stride, rv);
+        pool_body_velocity<KM>(B, v, col, stride, rv);
         TangentForce::gr_gradient(rp, rv, ir, ir2, B.mass, J);
         if (B.kind == FK_SUN && ng.kind != 0) TangentForce::nongrav_gradient(ng, rp, rv, ir, J, jp);
     }
@@ -95,7 +97,7 @@ __device__ __forceinline__ void pool_jacobian(const PoolTables& T, const double*
 }
 
 // The rounds of every group of the warp until the policies have no more work.
-template <int S, int THREADS, int TANGENTS, class Policy>
+template <int S, int THREADS, int TANGENTS, bool KM, class Policy>
 __device__ __forceinline__ void sens_pool_run(const PoolTables& T, double* smem, Policy& P,
                                               int max_rounds) {
     using Sh = SensPoolShared<S, THREADS, TANGENTS>;
@@ -198,8 +200,8 @@ __device__ __forceinline__ void sens_pool_run(const PoolTables& T, double* smem,
                 ste[lane] = __dmul_rn(te - 2451545.0, 86400.0);
             }
             __syncwarp();
-            pool_records<S, COLS, Sh::ROWS>(T, M, gi, ste, smem);
-            if (need && sub == 0) pool_chain(T, col, COLS);
+            pool_records<S, COLS, Sh::ROWS, KM>(T, M, gi, ste, smem);
+            if (need && sub == 0) pool_chain<KM>(T, col, COLS);
             __syncwarp();
             fresh = false;
         }
@@ -223,8 +225,8 @@ __device__ __forceinline__ void sens_pool_run(const PoolTables& T, double* smem,
         if (G.ng.kind != 0) {
             const PoolBody& sun = T.plan->b[0];
             double rp[3], rv[3];
-            pool_relative(xe, cl + sun.slot * COLS, COLS, rp);
-            pool_relative(ve, cl + sun.vslot * COLS, COLS, rv);
+            pool_body_position<KM>(sun, xe, cl, COLS, rp);
+            pool_body_velocity<KM>(sun, ve, cl, COLS, rv);
             const double3 p3 = make_double3(rp[0], rp[1], rp[2]), v3 = make_double3(rv[0], rv[1], rv[2]);
             const double3 r = (G.ng.kind == 1 && G.ng.p(9) == 0.0) ? nongrav_terms<false>(G.ng, p3, v3)
                                                                    : nongrav_accel(G.ng, p3, v3);
@@ -232,13 +234,13 @@ __device__ __forceinline__ void sens_pool_run(const PoolTables& T, double* smem,
         }
         if (S > 1) {
             const double own = sub == 0 ? na[0] : (sub == 1 ? na[1] : na[2]);
-            const double e = pool_forces_wide<true>(T.body, T.n_body, sub, cl, COLS, term, !iter_round,
-                                                    false, xe, ve, ex, own);
+            const double e = pool_forces_wide<true, KM>(T.body, T.n_body, sub, cl, COLS, term,
+                                                        !iter_round, false, xe, ve, ex, own);
             if (sub < 3) se[NODE_G * sub + lane] = e;
         } else {
             double ev[3];
-            pool_forces<true>(T.plan->b, T.n_vel, T.n_body, cl, COLS, !iter_round, false, xe, ve, ex,
-                              ev, na);
+            pool_forces<true, KM>(T.plan->b, T.n_vel, T.n_body, cl, COLS, !iter_round, false, xe, ve,
+                                  ex, ev, na);
             se[lane] = ev[0];
             se[NODE_G + lane] = ev[1];
             se[2 * NODE_G + lane] = ev[2];
@@ -494,7 +496,7 @@ struct SensPoolForward {
     }
 };
 
-template <int S, int THREADS, int MINB>
+template <int S, int THREADS, int MINB, bool KM>
 __global__ void __launch_bounds__(THREADS, MINB) sens_pool_forward_kernel(SensArgs a) {
     extern __shared__ __align__(16) double s_pool[];
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
@@ -502,7 +504,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sens_pool_forward_kernel(SensAr
     __shared__ PoolBody s_body[MAX_FORCE + 2];
     const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
     SensPoolForward P{a, ((int64_t)blockIdx.x * THREADS + threadIdx.x) / (NODE_G * S)};
-    sens_pool_run<S, THREADS, 0>(T, s_pool, P, a.max_loops * 12);
+    sens_pool_run<S, THREADS, 0, KM>(T, s_pool, P, a.max_loops * 12);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -622,7 +624,7 @@ struct SensPoolReplay {
     }
 };
 
-template <int S, int THREADS, int MINB>
+template <int S, int THREADS, int MINB, bool KM>
 __global__ void __launch_bounds__(THREADS, MINB) sens_pool_replay_kernel(SensArgs a) {
     extern __shared__ __align__(16) double s_pool[];
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
@@ -630,7 +632,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sens_pool_replay_kernel(SensArg
     __shared__ PoolBody s_body[MAX_FORCE + 2];
     const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
     SensPoolReplay P{a, a.rep_first[a.n]};
-    sens_pool_run<S, THREADS, 0>(T, s_pool, P, a.max_loops * 12);
+    sens_pool_run<S, THREADS, 0, KM>(T, s_pool, P, a.max_loops * 12);
 }
 
 // ---------------------------------------------------------------------------------------
@@ -638,6 +640,7 @@ __global__ void __launch_bounds__(THREADS, MINB) sens_pool_replay_kernel(SensArg
 // the four sub-lanes of a node take two of the eight directions each, the 24 rows of db and of
 // the state tangents a lane each.
 // ---------------------------------------------------------------------------------------
+template <bool KM>
 struct SensPoolStm {
     const StmArgs& a;
     int64_t obj;
@@ -646,8 +649,7 @@ struct SensPoolStm {
     double J[18], jp[6];  // the node's Jacobian at the last corrector iteration's point
 
     // da = J (dx, dv) + jp at the state, component sub and direction lane
-    __device__ void tangent_acc(SensPoolGroup& G, const double* col, const double Jn[18],
-                                const double jn[6]) {
+    __device__ void tangent_acc(SensPoolGroup& G, const double Jn[18], const double jn[6]) {
         double* ts = G.tan;
         const int p = G.lane;
 #pragma unroll
@@ -666,7 +668,7 @@ struct SensPoolStm {
     __device__ void state_jacobian(SensPoolGroup& G, const double* col, double Jn[18], double jn[6]) {
         const double x[3] = {G.st[ST_X], G.st[ST_X + 1], G.st[ST_X + 2]};
         const double v[3] = {G.st[ST_V], G.st[ST_V + 1], G.st[ST_V + 2]};
-        pool_jacobian(*G.T, col, G.stride, G.ng, x, v, Jn, jn);
+        pool_jacobian<KM>(*G.T, col, G.stride, G.ng, x, v, Jn, jn);
     }
     __device__ bool next(SensPoolGroup& G, bool&, int& failures, bool&) {
         if (!first || obj >= a.n) return false;
@@ -713,7 +715,7 @@ struct SensPoolStm {
             for (int i = threadIdx.x & 31; i < 168; i += 32) G.tan[STM_DB + i] = 0.0;
             double Jn[18], jn[6];
             state_jacobian(G, G.col, Jn, jn);
-            tangent_acc(G, G.col, Jn, jn);
+            tangent_acc(G, Jn, jn);
         }
         return true;
     }
@@ -723,7 +725,7 @@ struct SensPoolStm {
         __syncwarp(G.gmask);
     }
     __device__ void last_iteration(SensPoolGroup& G, const double*, const double* xe, const double* ve) {
-        pool_jacobian(*G.T, G.col, G.stride, G.ng, xe, ve, J, jp);
+        pool_jacobian<KM>(*G.T, G.col, G.stride, G.ng, xe, ve, J, jp);
     }
     __device__ void end_attempt(SensPoolGroup& G, int M, bool converged) {
         double* ts = G.tan;
@@ -797,7 +799,7 @@ struct SensPoolStm {
         __syncwarp(G.gmask);
         double Jn[18], jn[6];  // da' from the Jacobian at the accepted state
         state_jacobian(G, G.col_end, Jn, jn);
-        tangent_acc(G, G.col_end, Jn, jn);
+        tangent_acc(G, Jn, jn);
     }
     __device__ bool segment_end(SensPoolGroup& G, int&, bool&) {
         int rc = ST_OK;
@@ -826,15 +828,15 @@ struct SensPoolStm {
     }
 };
 
-template <int MINB>
+template <int MINB, bool KM>
 __global__ void __launch_bounds__(WIDE_BLOCK, MINB) sens_pool_stm_kernel(StmArgs a) {
     extern __shared__ __align__(16) double s_pool[];
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
     __shared__ PoolSeries s_src[MAX_SERIES];
     __shared__ PoolBody s_body[MAX_FORCE + 2];
     const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
-    SensPoolStm P{a, (int64_t)blockIdx.x};
-    sens_pool_run<4, WIDE_BLOCK, STM_ROW>(T, s_pool, P, a.max_loops * 12);
+    SensPoolStm<KM> P{a, (int64_t)blockIdx.x};
+    sens_pool_run<4, WIDE_BLOCK, STM_ROW, KM>(T, s_pool, P, a.max_loops * 12);
 }
 
 }  // namespace kb
