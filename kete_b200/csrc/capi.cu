@@ -1293,7 +1293,11 @@ static int thermal_model(int model, int64_t n, const double* sun2obj, const doub
         a.bb_coef[b] = band_wavelength[b] < 10.0 ? 0.0 : 397.289171e17 / ((wl_um * wl_um) * wl_um);
     }
     for (int b = n_bands; b < MAX_BANDS; ++b) a.bb_k[b] = 1.0;
-    for (int b = 0; b < MAX_BANDS; ++b) a.bb_ksum += a.bb_k[b];
+    a.bb_kmin = a.bb_k[0];
+    for (int b = 0; b < MAX_BANDS; ++b) {
+        a.bb_ksum += a.bb_k[b];
+        a.bb_kmin = std::min(a.bb_kmin, a.bb_k[b]);
+    }
     a.have_zero_mags = zero_mags ? 1 : 0;
     a.wise_cc = wise_color_correction ? 1 : 0;
     a.facets = ds->facets;

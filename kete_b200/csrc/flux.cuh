@@ -96,7 +96,7 @@ struct NeatmArgs {
     double bb_k[MAX_BANDS];     // black body: exponent numerator 1.43877688e4 / wavelength_um
     double bb_coef[MAX_BANDS];  // 397.289171e17 / wavelength_um^3; 0 when wavelength < 10 nm and
                                 // for the bands beyond n_bands (their bb_k is 1)
-    double bb_ksum;             // sum of bb_k over all MAX_BANDS
+    double bb_ksum, bb_kmin;    // sum and least of bb_k over all MAX_BANDS
     int have_zero_mags;
     int wise_cc;
     const double* band_albedo;  // n_bands x n

@@ -575,9 +575,11 @@ __device__ __forceinline__ void wise_factors(double t, double l, double& d0, dou
 // geometries with four WISE bands 2.27 -> 1.44 ms, with two NEOS bands 1.24 -> 0.80): T = Tss cos^(1/4) and 1 / T
 // come from two reciprocal square roots, the bands' divisions from one reciprocal of their
 // product.  That holds while the exponentials' product stays below e^600 (the WISE and NEOS
-// bands at 30 K: e^311); facets colder than that for their bands take the plain form.
+// bands at 30 K: e^311) and no denominator vanishes (an infinite temperature, a band whose
+// exponential rounds to one: inv_ss is NaN there); other facets take the plain form, a division
+// a band.
 template <int NB, bool CC>
-static __device__ __noinline__ void thermal_facet_cold(const NeatmArgs& a, double temp, double seen,
+static __device__ __noinline__ void thermal_facet_plain(const NeatmArgs& a, double temp, double seen,
                                                        double (&th)[NB]) {
     double d[3], w4;
     if (CC) {
@@ -585,6 +587,7 @@ static __device__ __noinline__ void thermal_facet_cold(const NeatmArgs& a, doubl
         wise_factors(t, log(t), d[0], d[1], d[2], w4);
     }
     for (int b = 0; b < NB; ++b) {
+        if (a.bb_coef[b] == 0.0) continue;  // 0, also over a vanishing denominator
         const double em1 = exp(a.bb_k[b] / temp) - 1.0;
         const double ff = a.bb_coef[b] / (CC && b < 3 ? em1 * d[b < 3 ? b : 0] : em1);
         th[b] += seen * (CC && b == 3 ? ff * w4 : ff);
@@ -600,7 +603,7 @@ __device__ __forceinline__ void thermal_facet(const NeatmArgs& a, double tmp, do
     if (!(temp >= 30.0)) return;
     const double inv_t = w * inv_ss;
     if (!(a.bb_ksum * inv_t < 600.0)) {
-        thermal_facet_cold<NB, CC>(a, temp, seen, th);
+        thermal_facet_plain<NB, CC>(a, temp, seen, th);
         return;
     }
     double den[NB];
@@ -668,7 +671,9 @@ __global__ void __launch_bounds__(32 * THERMAL_WARPS, 8) thermal_kernel(NeatmArg
             s_geo[3 + c][g] = obs2obj[c] / obs2obj_r;
         }
         s_geo[6][g] = ss_temp;
-        s_geo[7][g] = 1.0 / ss_temp;  // used where the temperature is at least 30 K
+        // used where the temperature is at least 30 K; no facet is hotter than ss_temp
+        const double inv_ss = 1.0 / ss_temp;
+        s_geo[7][g] = a.bb_kmin * inv_ss > 1e-15 ? inv_ss : __longlong_as_double(0x7ff8000000000000LL);
         // FRM: cos(lat_facet - lat_sun) (frm_facet_temperature, frm.rs:19-30) expanded with
         // the facet's cos/sin of latitude from the table
         if (a.model == 1) {
