@@ -59,7 +59,7 @@ extern "C" {
 
 /* propagate_n_body modes */
 /* AUTO: by the object count (a warp per object up to 4,096, the warp-pooled forms above) until
- * kete_b200_set_launch_config installs a configuration, then that configuration */
+ * kete_b200_set_launch_config installs a configuration (whichever), then that configuration */
 #define KETE_B200_MODE_AUTO 0
 #define KETE_B200_MODE_THREAD 1  /* one object per thread, one launch per call */
 #define KETE_B200_MODE_NODES 2   /* eight lanes per object: the 7 Gauss-Radau nodes in parallel */
@@ -367,6 +367,9 @@ int kete_b200_fp64_probe(int64_t iters, double* tflops, float* ms);
  * lane groups take objects from a queue as they finish; thread_block: block size of the
  * one-object-per-thread kernel. */
 int kete_b200_set_launch_config(int nodes_variant, int nodes_refill, int thread_block);
+/* Back to the state before the first kete_b200_set_launch_config: none installed, the automatic
+ * mode and the allocation-free entry point pick by the object count. */
+int kete_b200_reset_launch_config(void);
 
 /* Bound on each object's Radau step loop, in step attempts, for every N-body entry point
  * (propagate_n_body, the sensitivity and adjoint passes, the FOV N-body branch and

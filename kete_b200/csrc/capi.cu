@@ -785,8 +785,8 @@ int nodes_variant_for(int variant, int n_force) {
     return variant;
 }
 
-// The form a call in the automatic mode runs while the launch configuration is the one the
-// library starts with.  All of them give the same results to the bit; which is faster was
+// The form a call in the automatic mode runs while no launch configuration is installed.  All of
+// these give the same results to the bit; which is faster was
 // measured on B200 with the main belt over one year (us):
 //   n            1    600   2368   4000   10000   64000
 //   wide       144    271    379    528    1150    6240
@@ -813,12 +813,6 @@ void nodes_window(int variant, int n_force, double& lo, double& hi) {
         lo = P.lo;
         hi = P.hi;
     }
-}
-
-// Whether the launch configuration is the one the library starts with.
-static bool launch_is_default() {
-    const LaunchConfig d;
-    return g_launch.nodes_variant == d.nodes_variant && g_launch.nodes_refill == d.nodes_refill;
 }
 
 // What the pooled kernels read besides the plan in constant memory (no columns where the plan
@@ -855,8 +849,8 @@ int noalloc_snapshot(int64_t n, int include_asteroids, int64_t center, NBodyArgs
     if ((rc = center_chain(center, a.chain))) return rc;
     a.n_force = n_force;
     cfg = g_launch;
-    cfg.nodes_variant = launch_is_default() ? auto_variant(n, n_force)
-                                            : nodes_variant_for(cfg.nodes_variant, n_force);
+    cfg.nodes_variant = cfg.installed ? nodes_variant_for(cfg.nodes_variant, n_force)
+                                      : auto_variant(n, n_force);
     plan.general_variant = nodes_variant_for(7, n_force);
     nodes_window(cfg.nodes_variant, n_force, plan.lo, plan.hi);
     set_pool(a, plan.lo, plan.hi);
@@ -1096,7 +1090,7 @@ int kete_b200_propagate_n_body(int64_t n, const double* pos, const double* vel, 
     if (mode == KETE_B200_MODE_THREAD) {
         if ((rc = launch_nbody_thread(a, g_launch.thread_block, st))) return rc;
     } else if (mode == KETE_B200_MODE_NODES || mode == KETE_B200_MODE_AUTO) {
-        const bool automatic = mode == KETE_B200_MODE_AUTO && launch_is_default();
+        const bool automatic = mode == KETE_B200_MODE_AUTO && !g_launch.installed;
         const int variant = automatic ? auto_variant(n, a.n_force)
                                       : nodes_variant_for(g_launch.nodes_variant, a.n_force);
         const bool refill = automatic ? variant >= 9 : g_launch.nodes_refill != 0;
@@ -1743,6 +1737,17 @@ int kete_b200_set_launch_config(int nodes_variant, int nodes_refill, int thread_
     g_launch.nodes_variant = nodes_variant;
     g_launch.nodes_refill = nodes_refill ? 1 : 0;
     g_launch.thread_block = thread_block;
+    g_launch.installed = 1;
+    return 0;
+}
+
+int kete_b200_reset_launch_config(void) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    const LaunchConfig d;
+    g_launch.nodes_variant = d.nodes_variant;
+    g_launch.nodes_refill = d.nodes_refill;
+    g_launch.thread_block = d.thread_block;
+    g_launch.installed = 0;
     return 0;
 }
 

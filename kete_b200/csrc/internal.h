@@ -125,6 +125,7 @@ int launch_nodes_wide(NBodyArgs a, int general_variant, cudaStream_t stream);
 
 // launch configuration chosen by the tuner (kete_b200_set_launch_config)
 struct LaunchConfig {
+    int installed = 0;      // 0: none installed, the automatic mode picks by the object count
     int nodes_variant = 7;  // node-kernel form (see launch_nbody_nodes); 7 measured fastest
     int nodes_refill = 0;   // 1: persistent grid with an object queue
     int thread_block = 128;

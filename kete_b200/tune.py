@@ -14,6 +14,7 @@ configuration on the caller's own inputs (device arrays) and installs the fastes
 
 Until a configuration is installed, the automatic mode picks by the object count (a warp per
 object up to 4,096, then variants 9 and 10 with the queue); the explicit mode runs variant 7.
+``set_config()`` goes back to that.
 """
 from __future__ import annotations
 
@@ -28,14 +29,26 @@ from .propagation import propagate_n_body_arrays
 CONFIGS = [dict(mode=_lib.MODE_NODES, variant=v, refill=r) for v, r in
            itertools.product((0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10), (0, 1))] + [
                dict(mode=_lib.MODE_THREAD, variant=0, refill=0)]
-_current = dict(mode=_lib.MODE_NODES, variant=7, refill=0, thread_block=128)
+_START = dict(mode=_lib.MODE_NODES, variant=7, refill=0, thread_block=128)
+_current = dict(_START, automatic=True)
 
 
-def set_config(mode=_lib.MODE_NODES, variant=7, refill=0, thread_block=128):
+def set_config(mode=None, variant=None, refill=None, thread_block=None, automatic=None):
+    """Install a launch configuration (what is not given: variant 7, no queue, blocks of 128),
+    or, without arguments or with automatic=True, go back to the automatic choice."""
+    given = {k: v for k, v in (("mode", mode), ("variant", variant), ("refill", refill),
+                               ("thread_block", thread_block)) if v is not None}
+    automatic = not given if automatic is None else bool(automatic)
+    cfg = dict(_START, **given)
     L = _lib.lib()
-    L.kete_b200_set_launch_config.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
-    _lib.check(L.kete_b200_set_launch_config(int(variant), int(refill), int(thread_block)))
-    _current.update(mode=mode, variant=variant, refill=refill, thread_block=thread_block)
+    if automatic:
+        cfg = dict(_START)
+        _lib.check(L.kete_b200_reset_launch_config())
+    else:
+        L.kete_b200_set_launch_config.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_int]
+        _lib.check(L.kete_b200_set_launch_config(int(cfg["variant"]), int(cfg["refill"]),
+                                                 int(cfg["thread_block"])))
+    _current.update(cfg, automatic=automatic)
 
 
 def set_step_limit(max_steps: int = 0):
