@@ -302,14 +302,23 @@ static void build_fast_plan(int n_force, FastPlan& P) {
 }
 
 // The pooled kernels' series and bodies (PoolPlan) of the fast plan P: the same bodies,
-// centres, segments and window, with each series' records appended to the pool.
-static void build_pool_plan(const FastPlan& P, PoolPlan& Q) {
+// centres, segments and window, with each series' records appended to the pool unless they are
+// there already (laid: SPK slot -> the series of an earlier plan).
+static void build_pool_plan(const FastPlan& P, PoolPlan& Q, std::map<int, PoolSeries>& laid) {
     std::memset(&Q, 0, sizeof Q);
     if (!P.ok) return;
     std::map<int, int> at;  // SPK slot -> its position series
     auto add_series = [&](int slot) {
         if (at.count(slot)) return at[slot];
         if (Q.n_pos >= MAX_SERIES) return -1;
+        const auto have = laid.find(slot);
+        if (have != laid.end()) {
+            Q.s[Q.n_pos] = have->second;
+            Q.s[Q.n_pos].slot = Q.n_slot;
+            Q.n_slot += 3;
+            at[slot] = Q.n_pos;
+            return Q.n_pos++;
+        }
         const SegDesc& d = g_eph.seg[g_eph.slot[slot].first];
         // trailing coefficients that are zero in every record (the padding of mixed counts)
         // are left out
@@ -331,7 +340,6 @@ static void build_pool_plan(const FastPlan& P, PoolPlan& Q) {
         S.rsize = 4 + 6 * pairs;
         S.pairs = pairs;
         S.slot = Q.n_slot;
-        g_pool_host.reserve(g_pool_host.size() + (size_t)d.n_rec * S.rsize);
         for (int64_t r = 0; r < d.n_rec; ++r) {
             const int64_t o = d.offset + r * d.rsize;
             for (int64_t k : {o, o + 2, o + 3}) g_pool_host.push_back(g_pool_host[k]);
@@ -342,6 +350,7 @@ static void build_pool_plan(const FastPlan& P, PoolPlan& Q) {
                         g_pool_host.push_back(g_pool_host[o + 4 + c * d.n_pad + k]);
         }
         Q.n_slot += 3;
+        laid[slot] = S;
         at[slot] = Q.n_pos;
         return Q.n_pos++;
     };
@@ -420,6 +429,15 @@ static int rebuild_tables() {
     for (const auto& sg : g_segs)
         if (sg.type == 2) max_coef = std::max<int64_t>(max_coef, sg.n_coef);
     const bool common_pad = max_coef <= FAST_NC;
+    // sized once: the general records, and of type 2 the pooled kernels' as well
+    size_t doubles = 0;
+    for (const auto& s : g_segs) {
+        const size_t pad = s.type == 2 && common_pad ? FAST_NC : (size_t)((s.n_coef + 1) & ~1LL);
+        if (s.type == 2) doubles += 2 * (size_t)s.n_rec * (4 + 3 * pad) + 1;
+        else if (s.type == 3) doubles += (size_t)s.n_rec * (4 + 6 * pad);
+        else doubles += (size_t)s.n_rec * (size_t)(s.rsize + 1);
+    }
+    g_pool_host.reserve(doubles);
     int nseg = 0;
     for (size_t si = 0; si < ids.size(); ++si) {
         Slot& sl = g_eph.slot[si];
@@ -537,8 +555,9 @@ static int rebuild_tables() {
     g_eph.n_force_all = (planets_ok && all_ok) ? N_MASSES : 0;
     build_fast_plan(g_eph.n_force_planets, g_eph.fast_planets);
     build_fast_plan(g_eph.n_force_all, g_eph.fast_all);
-    build_pool_plan(g_eph.fast_planets, g_plans.planets);
-    build_pool_plan(g_eph.fast_all, g_plans.all);
+    std::map<int, PoolSeries> laid;
+    build_pool_plan(g_eph.fast_planets, g_plans.planets, laid);
+    build_pool_plan(g_eph.fast_all, g_plans.all, laid);
     g_eph.sun_slot = g_slot_of.count(10) ? g_slot_of[10] : -1;
     g_eph.loaded = 1;
     ++g_version;
