@@ -343,9 +343,8 @@ constexpr int ORDER_BLOCK = 256;
 // Bucket starts (the cursors) and the range from the histogram: one block, one bucket a thread.
 //
 // groups > 0 (a persistent pooled launch with that many lane groups): the objects of the classes
-// whose work is over HEAVY_SHARE of a group's share of all the work would still run when the
-// others are done; the pooled kernel gives them a warp each (at most half its warps' worth).
-constexpr float HEAVY_SHARE = 1.0f;
+// whose work is over a group's share of all the work would still run when the others are done;
+// the pooled kernel gives them a warp each (at most half its warps' worth).
 __global__ void __launch_bounds__(ORDER_BLOCK) order_scan_kernel(int groups,
                                                                  int* __restrict__ scratch) {
     __shared__ int start[ORDER_BLOCK];
@@ -375,7 +374,7 @@ __global__ void __launch_bounds__(ORDER_BLOCK) order_scan_kernel(int groups,
     if (t < ORDER_OUT_BUCKET) atomicAdd(&total, (float)own * work * 1.09f);
     __syncthreads();
     if (t == 0 || t == ORDER_NG_BUCKET) {
-        const float limit = HEAVY_SHARE * total / (float)groups;
+        const float limit = total / (float)groups;
         const int most = groups / 16;  // of each part: a quarter of the warps
         int heavy = 0;
         for (int c = 0; c < ORDER_CLASSES; ++c) {

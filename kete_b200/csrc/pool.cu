@@ -23,11 +23,11 @@ static const void* kernel_ptr(int variant, bool km) {
         case NODES_WIDE:
             return km ? (const void*)nbody_wide_kernel<16, true> : (const void*)nbody_wide_kernel<16, false>;
         case 9:
-            return km ? (const void*)nbody_pool_kernel<3, true, true>
-                      : (const void*)nbody_pool_kernel<3, true, false>;
+            return km ? (const void*)nbody_pool_kernel<3, true>
+                      : (const void*)nbody_pool_kernel<3, false>;
         default:
-            return km ? (const void*)nbody_pool_kernel<4, true, true>
-                      : (const void*)nbody_pool_kernel<4, true, false>;
+            return km ? (const void*)nbody_pool_kernel<4, true>
+                      : (const void*)nbody_pool_kernel<4, false>;
     }
 }
 const void* pool_kernel_ptr(int variant) { return kernel_ptr(variant, false); }
@@ -71,13 +71,13 @@ int launch_pool(const NBodyArgs& a, int variant, int grid, cudaStream_t stream) 
     else if (variant == NODES_WIDE)
         nbody_wide_kernel<16, false><<<grid, WIDE_BLOCK, smem, stream>>>(a);
     else if (variant == 9 && a.pool_km)
-        nbody_pool_kernel<3, true, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
+        nbody_pool_kernel<3, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
     else if (variant == 9)
-        nbody_pool_kernel<3, true, false><<<grid, NODES_BLOCK, smem, stream>>>(a);
+        nbody_pool_kernel<3, false><<<grid, NODES_BLOCK, smem, stream>>>(a);
     else if (a.pool_km)
-        nbody_pool_kernel<4, true, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
+        nbody_pool_kernel<4, true><<<grid, NODES_BLOCK, smem, stream>>>(a);
     else
-        nbody_pool_kernel<4, true, false><<<grid, NODES_BLOCK, smem, stream>>>(a);
+        nbody_pool_kernel<4, false><<<grid, NODES_BLOCK, smem, stream>>>(a);
     return launched(1, "nbody_pool_kernel launch");
 }
 

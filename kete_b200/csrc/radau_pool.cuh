@@ -1036,22 +1036,20 @@ __device__ __forceinline__ PoolTables pool_tables(int n_force, double* s_node,
 // 128); the host picks the instantiation.  With a.queue the grid is persistent and groups take
 // objects from the queues; without, each group integrates one object.
 //
-// HEAVY: the first blocks begin with the order's heavy objects, a warp each, and turn to the
-// others when those are taken.  The objects with many times the steps of most (near the Earth,
-// long spans) bound a launch of a few objects per lane group: see order_scan_kernel for the
-// rule.
-template <int MINB, bool HEAVY, bool KM>
+// The first blocks begin with the order's heavy objects, a warp each, and turn to the others when
+// those are taken (without any, the counts are zero).  The objects with many times the steps of
+// most (near the Earth, long spans) bound a launch of a few objects per lane group: see
+// order_scan_kernel for the rule.
+template <int MINB, bool KM>
 __global__ void __launch_bounds__(NODES_BLOCK, MINB) nbody_pool_kernel(NBodyArgs a) {
     extern __shared__ __align__(16) double s_pool[];
     __shared__ __align__(16) double s_node[9 * POOL_NODE];
     __shared__ PoolSeries s_src[MAX_SERIES];
     __shared__ PoolBody s_body[MAX_FORCE + 2];
     const PoolTables T = pool_tables(a.n_force, s_node, s_src, s_body);
-    if (HEAVY) {
-        if ((int)blockIdx.x * (NODES_BLOCK / 32) < a.wide[0] + a.wide[1])
-            pool_run<4, NODES_BLOCK, true, KM>(a, T, s_pool);
-        __syncthreads();
-    }
+    if ((int)blockIdx.x * (NODES_BLOCK / 32) < a.wide[0] + a.wide[1])
+        pool_run<4, NODES_BLOCK, true, KM>(a, T, s_pool);
+    __syncthreads();
     pool_run<1, NODES_BLOCK, true, KM>(a, T, s_pool);
 }
 
