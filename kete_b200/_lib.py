@@ -85,6 +85,17 @@ def _is_torch_cuda(a) -> bool:
     return getattr(a, "is_cuda", False) and type(a).__module__.startswith("torch")
 
 
+def _current_stream(device: int) -> int:
+    """Handle of torch's current stream: the raw one, where this torch has it, since
+    torch.cuda.current_stream wraps it in a Stream (4 us)."""
+    import torch
+
+    try:
+        return torch._C._cuda_getCurrentRawStream(device)
+    except AttributeError:
+        return torch.cuda.current_stream(device).cuda_stream
+
+
 class Args:
     """Collects array pointers for one call; all arrays must live on the same side."""
 
@@ -103,10 +114,7 @@ class Args:
             if not a.is_contiguous():
                 raise ValueError("device arrays must be contiguous")
             if self.stream is None:
-                import torch
-
-                # the raw handle: torch.cuda.current_stream wraps it in a Stream (4 us)
-                self.stream = torch._C._cuda_getCurrentRawStream(a.get_device())
+                self.stream = _current_stream(a.get_device())
             self.keep.append(a)
             return a.data_ptr()
         if self.device is True:
