@@ -73,10 +73,8 @@ static int launch_sens_pass(SensArgs a, bool passes, cudaStream_t stream) {
     if (a.pending && (rc = launch_sens_pool_replay(a, stream))) return rc;
     // persistent grid: as many thread blocks as are resident at once, and no more than the
     // blocks to replay could occupy
-    int dev = 0, sms = 0, per_sm = 0;
-    if ((rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice")) ||
-        (rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
-                         "attr")) ||
+    int sms = 0, per_sm = 0;
+    if ((rc = sm_count(&sms)) ||
         (rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
                              &per_sm, nbody_sens_replay_kernel<3>, SENS_BLOCK, cache_bytes),
                          "occupancy")))

@@ -28,6 +28,14 @@ inline cudaError_t counted_malloc(void** p, size_t bytes) {
     return e;
 }
 
+// SMs of the current device
+inline int sm_count(int* sms) {
+    int dev = 0;
+    const int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    if (rc) return rc;
+    return cuda_check(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev), "SM count");
+}
+
 // every launch helper adds the kernels it enqueued when it checks the launch
 inline int launched(int kernels, const char* what) {
     g_kernel_launches.fetch_add(kernels, std::memory_order_relaxed);

@@ -761,9 +761,13 @@ __global__ void __launch_bounds__(32 * THERMAL_WARPS, 8) thermal_kernel(NeatmArg
 
 int launch_neatm(const NeatmArgs& a, cudaStream_t stream) {
     if (a.n <= 0) return 0;
-    // a warp per geometry until the GPU is full of them, then up to THERMAL_MAX a block
+    // a warp per geometry until the GPU is full of them (8 blocks an SM) twice, then up to
+    // THERMAL_MAX a block
+    int sms = 0;
+    const int rc = sm_count(&sms);
+    if (rc) return rc;
     int per_block = THERMAL_WARPS;
-    while (per_block < THERMAL_MAX && a.n >= (int64_t)per_block * 148 * 8 * 2) per_block *= 2;
+    while (per_block < THERMAL_MAX && a.n >= (int64_t)per_block * sms * 8 * 2) per_block *= 2;
     const unsigned grid = (unsigned)((a.n + per_block - 1) / per_block);
     const unsigned block = 32 * THERMAL_WARPS;
     if (a.wise_cc)  // the capi admits colour corrections only with the 4 WISE bands

@@ -129,11 +129,9 @@ int preload_nodes_kernels() {
 
 // Resident grid for the persistent (refill) form: blocks per SM from the occupancy API.
 int nodes_grid_size(int variant, int slots, int* grid) {
-    int dev = 0, sms = 0, per_sm = 0;
-    int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    int sms = 0, per_sm = 0;
+    int rc = sm_count(&sms);
     if (rc) return rc;
-    if ((rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")))
-        return rc;
     int smem = 0;
     if (variant >= 9 && (rc = pool_smem(variant, slots, &smem))) return rc;
     if ((rc = cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(

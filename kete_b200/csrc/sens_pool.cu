@@ -36,17 +36,20 @@ using Shared1 = SensPoolShared<1, SENS_POOL_BLOCK, 0>;
 using Shared4 = SensPoolShared<4, WIDE_BLOCK, 0>;
 using SharedStm = SensPoolShared<4, WIDE_BLOCK, STM_ROW>;
 
-// A warp per object while one wave of blocks (12 per SM of 148) takes them all, eight lanes above:
-// what counts is then the slowest object's chain of steps, afterwards how many run at a time.
+// A warp per object while one wave of blocks (12 per SM) takes them all (1,776 on 148 SMs), eight
+// lanes above: what counts is then the slowest object's chain of steps, afterwards how many run at a time.
 // Measured, 400 days: 50 objects 2.87 ms and 3.73, 1000 objects 3.66 and 4.49, 2048 objects 5.05
 // and 4.45; 730 days, 4096 objects: 14.06 and 8.96 (thread groups that replay per node: 12.8).
-constexpr int64_t SENS_WIDE_MAX = 1776;
+constexpr int SENS_WIDE_PER_SM = 12;
 
 template <bool KM>
 static int launch_forward(const SensArgs& a, cudaStream_t stream) {
-    if (a.n <= SENS_WIDE_MAX) {
+    int sms = 0;
+    const int src = sm_count(&sms);
+    if (src) return src;
+    if (a.n <= (int64_t)SENS_WIDE_PER_SM * sms) {
         const int smem = Shared4::doubles(a.pool_slots) * (int)sizeof(double);
-        sens_pool_forward_kernel<4, WIDE_BLOCK, 12, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
+        sens_pool_forward_kernel<4, WIDE_BLOCK, SENS_WIDE_PER_SM, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
     } else {
         const auto kernel = sens_pool_forward_kernel<1, SENS_POOL_BLOCK, 3, KM>;
         const int smem = Shared1::doubles(a.pool_slots) * (int)sizeof(double);
@@ -66,10 +69,9 @@ int launch_sens_pool_forward(const SensArgs& a, cudaStream_t stream) {
 // Persistent grids; a.n * a.window bounds the blocks to replay.
 template <bool KM>
 static int launch_replay(const SensArgs& a, cudaStream_t stream) {
-    int dev = 0, sms = 0, per_sm = 0;
-    int rc = cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-    if (rc || (rc = cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "attr")))
-        return rc;
+    int sms = 0, per_sm = 0;
+    int rc = sm_count(&sms);
+    if (rc) return rc;
     const int64_t most = a.n * (int64_t)a.window;
     const bool wide = most <= 8192;
     const auto k4 = sens_pool_replay_kernel<4, WIDE_BLOCK, 12, KM>;
@@ -102,7 +104,10 @@ static int launch_stm(const StmArgs& a, cudaStream_t stream) {
     // Eight blocks an SM leave a thread 255 registers, which pays while that is one wave: 1021
     // objects 6.46 ms and 6.81 with twelve, 4096 objects 38.8 ms and 34.3
     // (sixteen: 38.4).
-    if (a.n <= 8 * 148) sens_pool_stm_kernel<8, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
+    int sms = 0;
+    const int rc = sm_count(&sms);
+    if (rc) return rc;
+    if (a.n <= (int64_t)8 * sms) sens_pool_stm_kernel<8, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
     else sens_pool_stm_kernel<12, KM><<<(unsigned)a.n, WIDE_BLOCK, smem, stream>>>(a);
     return launched(1, "sens_pool_stm_kernel launch");
 }
