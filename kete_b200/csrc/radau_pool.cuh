@@ -307,6 +307,35 @@ __device__ __forceinline__ void pool_forces(const PoolBody* body, int n_vel, int
     }
 }
 
+// A struck body ends the list of those that count, for the impact (the first of the plan) as for the
+// closest approach.  The sub-lanes of a node, each of which saw its own bodies, go through all of
+// them again here in the plan's order, as pool_forces does.
+template <bool KM>
+__device__ __forceinline__ PoolExact pool_impact(const PoolBody* body, int n_body, const double* col,
+                                                     int stride, bool exact, bool track, double x0,
+                                                     double x1, double x2, double min_before) {
+    const double x[3] = {x0, x1, x2};
+    PoolExact ex;
+    ex.impact_id = 0;
+    ex.min_r2 = min_before;
+#pragma unroll 1
+    for (int i = 0; i < n_body; ++i) {
+        double rp[3];
+        pool_body_position<KM>(body[i], x, col, stride, rp);
+        pool_checks(body[i], pool_r2(rp), exact, track, ex);
+    }
+    return ex;
+}
+
+// Out of line for the planets (one object over a year 207 -> 202 us); with the asteroids' longer
+// plan the call costs the pooled kernel spills (9,973 objects over two years 3.62 -> 3.64 ms).
+static __device__ __noinline__ PoolExact pool_impact_planets(const PoolBody* body, int n_body,
+                                                             const double* col, int stride, bool exact,
+                                                             bool track, double x0, double x1, double x2,
+                                                             double min_before) {
+    return pool_impact<false>(body, n_body, col, stride, exact, track, x0, x1, x2, min_before);
+}
+
 // The same sum by the four sub-lanes of a node, to the bit: every sub-lane forms the scalars
 // of its bodies (the Sun or Jupiter, and pairs of the others), then sub-lane c adds up
 // component c in the plan's order.  term: the warp's scalars, slot k of a node at k * NODE_G.
@@ -357,18 +386,15 @@ __device__ __forceinline__ double pool_forces_wide(const PoolBody* body, int n_b
             term[(TERM_EARTH + 1) * NODE_G] = z2;
         }
     }
-    // A struck body ends the list of those that count, for the impact (the first of the plan) as for
-    // the closest approach: the sub-lanes, each of which saw its own bodies, go through all of them
-    // again in the plan's order, as pool_forces does.
     if (__any_sync(0xffffffffu, ex.impact_id != 0)) {
-        ex.impact_id = 0;
-        ex.min_r2 = min_before;
-#pragma unroll 1
-        for (int i = 0; i < n_body; ++i) {
-            double rp[3];
-            pool_body_position<KM>(body[i], x, col, stride, rp);
-            pool_checks(body[i], pool_r2(rp), exact, track, ex);
-        }
+        if (NG_SUN)  // the differentiation passes ask whether, not which
+#pragma unroll
+            for (int o = NODE_G; o < 32; o <<= 1)
+                ex.impact_id = max(ex.impact_id, __shfl_xor_sync(0xffffffffu, ex.impact_id, o));
+        else if (KM)
+            ex = pool_impact<true>(body, n_body, col, stride, exact, track, x[0], x[1], x[2], min_before);
+        else
+            ex = pool_impact_planets(body, n_body, col, stride, exact, track, x[0], x[1], x[2], min_before);
     }
     if (track)
 #pragma unroll
