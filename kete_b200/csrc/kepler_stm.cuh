@@ -20,7 +20,9 @@ namespace kb {
 
 // g0 .. g5 of the universal functions at anomaly s (g_k = s^k c_k(z), z = beta s^2, Stumpff
 // functions), given g1 and g2 of the same beta.  For |z| < 0.1 g3 .. g5 come from the
-// alternating series, which stays accurate where (s - g1) / beta and its successors cancel.
+// alternating series, which stays accurate where (s - g1) / beta and its successors cancel, and
+// g1 and g2 from those by g_k = s^k / k! - beta g_(k+2): the solver's hyperbolic (1 - cosh) / beta
+// cancels too (at perihelion, beta = -3e-8, an eighth of a day: 3e-10 of a block of the matrix).
 struct Universal {
     double g0, g1, g2, g3, g4, g5;
 };
@@ -47,6 +49,9 @@ __device__ __forceinline__ Universal universal_functions(double s, double beta, 
         u.g3 = s2 * s * c3;
         u.g4 = s2 * s2 * c4;
         u.g5 = s2 * s2 * s * c5;
+        u.g2 = 0.5 * s2 - beta * u.g4;
+        u.g1 = s - beta * u.g3;
+        u.g0 = 1.0 - beta * u.g2;
         return u;
     }
     const double ib = 1.0 / beta;
