@@ -15,8 +15,9 @@
 // says which: these kernels or the pooled ones of sens_pool.cuh, whose sums may round otherwise;
 // another rounding changes which attempts are retried, and a block of so many attempts would
 // end elsewhere than the next begins), recording for every attempt its start state, the step
-// size used, its iteration count and the b of its last corrector iteration.  The attempts are then transposed, last first.  For one attempt
-// with M iterations (step size and iteration count held fixed):
+// size used, its iteration count and the b of its last corrector iteration.  The attempts are then
+// transposed, last first.  For one attempt with M iterations (step size and iteration count held
+// fixed):
 //   x' = x + h v + h^2 (a/2 + W.b^M),  v' = v + h (a + U.b^M),  a' = F(x', v')
 //   b^m = P (E^m - a),  E^m_j = F(X_j(b^(m-1)), V_j(b^(m-1))),  P = C_MAT . (divided differences)
 //   b^0 = S(q) b^M of the previous attempt (the predictor, q = h / h_prev; identity after a
@@ -530,8 +531,8 @@ static __device__ __noinline__ int sens_jacobian(TangentForce& T, double t, cons
 // Re-run checkpoint block `c` (its segment ends at tf; next: the checkpoint it leads to, null for
 // the last block) with the step code, recording every attempt into rec (SENS_CK_ATTEMPTS + 1
 // records).  Returns ST_OK with the attempt count in na, or the failure.
-__device__ __forceinline__ int sens_replay_block(const double* c, double tf, const double* next, double* rec,
-                                                 SpkForce& F, const double* nrow, double* sb,
+__device__ __forceinline__ int sens_replay_block(const double* c, double tf, const double* next,
+                                                 double* rec, SpkForce& F, const double* nrow, double* sb,
                                                  double* se, int lane, int comp, unsigned gmask,
                                                  int warp_lane, int max_rounds, EphCache& C,
                                                  int& na) {
@@ -628,8 +629,9 @@ __global__ void __launch_bounds__(SENS_BLOCK, MINB) nbody_sens_replay_kernel(Sen
         double* rec = a.rec_all + (size_t)item * (SENS_CK_ATTEMPTS + 1) * SENS_STRIDE;
         const double* c = a.ckpt + ((size_t)obj * a.ckpt_cap + cb) * SENS_STRIDE;
         int na = 0;
-        const int rc = sens_replay_block(c, a.epochs[k], sens_next_checkpoint(a, obj, k, cb), rec, F, nrow, sb, se, lane, comp, gmask,
-                                         warp_lane, a.max_loops * 12, C, na);
+        const int rc = sens_replay_block(c, a.epochs[k], sens_next_checkpoint(a, obj, k, cb), rec, F,
+                                         nrow, sb, se, lane, comp, gmask, warp_lane,
+                                         a.max_loops * 12, C, na);
         if (lane == 0) a.rep_count[item] = rc == ST_OK ? na : -1 - rc;
         __syncwarp(gmask);  // sb, se and the cache are reused by the group's next block
     }

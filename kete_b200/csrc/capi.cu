@@ -804,9 +804,9 @@ int nodes_variant_for(int variant, int n_force) {
     return variant;
 }
 
-// The form a call in the automatic mode runs while no launch configuration is installed.  All of
-// these give the same results to the bit; which is faster was
-// measured on B200 with the main belt over one year (us):
+// The form a call in the automatic mode runs while no launch configuration is installed.  These
+// three (not the others) give the same results to the bit; which is faster was measured on B200
+// with the main belt over one year (us):
 //   n            1    600   2368   4000   10000   64000
 //   wide       144    271    379    528    1150    6240
 //   variant 9  197    456    475    579     746    3533   (168 registers, refill)

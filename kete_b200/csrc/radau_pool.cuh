@@ -15,11 +15,12 @@
 // The integration of each object is the one of radau_nodes.cuh with the step-end lane
 // (lane 7 evaluates the step end during each corrector iteration and supplies the exact
 // evaluation of the accepted step), the predicted corrector start and the compensated state
-// update, in the same arithmetic: objects without a non-gravitational model get the results of
-// the other cached forms to the bit but for one in two thousand, and keep them when the work
-// is split otherwise.  That matters beyond tidiness: the corrector's 1e-14 test lies in the
-// rounding noise of b6, so a different rounding anywhere changes which steps are retried, and
-// close approaches amplify that from 1e-11 AU to 1e-6 and more.
+// update, in the same arithmetic.  Every form in this file (variants 9 and 10 with and without the
+// queue, a warp per object) gives an object the same results to the bit; with the planets,
+// objects without a non-gravitational model get those of the cached variants 6 to 8
+// (radau_nodes.cuh) to the bit but for one in two thousand.  That matters beyond tidiness: the
+// corrector's 1e-14 test lies in the rounding noise of b6, so a different rounding anywhere changes
+// which steps are retried, and close approaches amplify that from 1e-11 AU to 1e-6 and more.
 //
 // What bounds it (100,000 objects of the +-5 yr mix, ncu): the L1 data pipe, 72% of the active
 // cycles -- about half of its wavefronts are the record loads (each lane reads its own
