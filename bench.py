@@ -1677,8 +1677,8 @@ def run_stm(args, world, rank, local):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": (achieved / peak) if peak else None, "traffic": None,
                      "bytes_per_object": STM_BYTES_PER_OBJECT,
-                     "note": "algorithmic bytes over the kernel time; the dual-number leaf "
-                             "Jacobians make it FP64/latency-bound (ncu: 31.6% FP64 pipe)"},
+                     "note": "algorithmic bytes over the call's time; bound by the loads and "
+                             "stores of its 123 columns a thread (ncu: 39% FP64 pipe)"},
         "cpu_baseline": {"value": k / cpu_s, "unit": "objects/s", "cores": 1, "kind": "port",
                          "sample": f"the first {k} objects, one thread"},
         "e2e": {"value": world * n / e2e_s, "unit": "objects/s",
